@@ -172,6 +172,57 @@ def work(case):
     }
 
 
+def _dequant_weight(w, scale):
+    """One expert's weight in 64 bits; fp8: every 128x128 block times its scale."""
+    if scale is None:
+        return w.double()
+    blocks = scale.double().repeat_interleave(128, 0)[: w.shape[0]].repeat_interleave(128, 1)[:, : w.shape[1]]
+    return w.to(torch.float32).double() * blocks
+
+
+def _quantised(x):
+    """Activations as the fp8 path defines them: e4m3 with one scale per row and 128 columns,
+    a power of two where the reference's quantiser makes it one."""
+    groups = x.reshape(x.shape[0], -1, 128)
+    scale = groups.abs().amax(-1, keepdim=True).clamp(min=1e-10) / 448.0
+    if capi.reference_fp8_scale_format() == "ue8m0":
+        scale = torch.exp2(torch.ceil(torch.log2(scale)))
+    q = (groups / scale).clamp(-448.0, 448.0).float().to(torch.float8_e4m3fn)
+    return (q.float().double() * scale).reshape(x.shape)
+
+
+def exact(case, seed):
+    """What ``run`` returns, in 64 bits: the router's ids and weights, or the layer's output,
+    expert by expert (fp8: on the quantised activations that the precision means)."""
+    if case["entry"] == "router":
+        logits = prepare(case, seed)["logits"].double()
+        best, ids = torch.sort(logits, dim=1, descending=True, stable=True)
+        best, ids = best[:, : case["topk"]], ids[:, : case["topk"]]
+        return ids.to(torch.int32), torch.softmax(best, 1)
+    problem = make_problem(_config(case, seed), case["tokens"])
+    fp8 = case["precision"] == "fp8"
+    x = problem.hidden_states.double()
+    if fp8:
+        x = _quantised(x)
+    ids = problem.topk_ids.long()
+    if problem.expert_map is not None:
+        ids = problem.expert_map.long()[ids]
+    out = torch.zeros_like(x)
+    n = problem.w1.shape[1] // 2
+    for e in range(problem.w1.shape[0]):
+        token, slot = torch.nonzero(ids == e, as_tuple=True)
+        if token.numel() == 0:
+            continue
+        w1 = _dequant_weight(problem.w1[e], problem.quant_config.w1_scale[e] if fp8 else None)
+        w2 = _dequant_weight(problem.w2[e], problem.quant_config.w2_scale[e] if fp8 else None)
+        h = x[token] @ w1.t()
+        act = torch.nn.functional.silu(h[:, :n]) * h[:, n:]
+        if fp8:
+            act = _quantised(act.bfloat16().double())  # bf16 activations are part of the precision
+        out.index_add_(0, token, problem.topk_weights[token, slot].double()[:, None] * (act @ w2.t()))
+    return out
+
+
 def tolerance(case):
     if case["entry"] == "router":
         # fp32 softmax over a few selected logits; the ids are exact

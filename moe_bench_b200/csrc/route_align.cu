@@ -2,8 +2,8 @@
 //
 //  * route_topk: softmax over the expert logits, top-k selection, weights
 //    renormalised over the selected experts.  One warp per token; the selection
-//    is k rounds of a warp-shuffle arg-max (largest logit first, lowest expert
-//    index wins ties).  The reference has no router (data.py:178-235 draws the
+//    is k rounds of a warp arg-max on ordered integer keys (largest logit first,
+//    lowest expert index wins ties).  The reference has no router (data.py:178-235 draws the
 //    ids directly); this is the front end a caller with logits needs.
 //
 //  * align: stable counting sort of the flat assignment index n = token*k+kpos
@@ -23,8 +23,29 @@ namespace mb200 {
 namespace {
 
 // ---------------------------------------------------------------- route_topk
-constexpr int kRouteMaxPerLane = 32;  // experts <= 1024
+constexpr int kRouteMaxExperts = 1024;
 
+// Order-preserving image of a logit in uint32: larger logit <-> larger key, -0 == +0.
+// NaN maps to 0, below the key of -inf: a NaN logit is never selected.
+__device__ __forceinline__ uint32_t logit_key(float v) {
+  const uint32_t u = __float_as_uint(v + 0.0f);  // -0 + 0 = +0
+  const uint32_t key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+  return v != v ? 0u : key;
+}
+__device__ __forceinline__ float key_logit(uint32_t key) {
+  if (key == 0u) return -INFINITY;  // nothing but NaN in the row
+  return __uint_as_float((key & 0x80000000u) ? (key ^ 0x80000000u) : ~key);
+}
+constexpr uint32_t kKeyNegInf = 0x007FFFFFu;  // logit_key(-inf)
+
+// One warp per token, lane l holds experts l, l+32, ... (coalesced loads) as ordered integer
+// keys.  Instruction issue bounds this kernel (the 8 MB of logits are two microseconds of HBM), so
+// the k rounds are kept short: each lane caches its own best (key, expert); a round is two warp
+// reductions (redux.sync: largest key, then lowest expert among the lanes that hold it) and a
+// rescan of kPerLane registers after the winner is retired.  kPerLane is a template parameter so
+// that the rescan has exactly as many steps as the expert count needs.  8192 x 256 logits, top-8:
+// 12.3 us against 41.0 us with ten shuffles and 32 predicated compares per round.
+template <int kPerLane>
 __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, int experts,
                                   int topk, int* __restrict__ ids, float* __restrict__ weights) {
   const int warps_per_block = blockDim.x >> 5;
@@ -33,63 +54,58 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, 
   if (token >= tokens) return;
   const float* row = logits + size_t(token) * experts;
 
-  // lane l holds experts l, l+32, ... (coalesced loads)
-  float v[kRouteMaxPerLane];
-  const int per_lane = (experts + 31) >> 5;
-  float mx = -INFINITY;
+  uint32_t key[kPerLane];
 #pragma unroll
-  for (int i = 0; i < kRouteMaxPerLane; ++i) {
-    if (i < per_lane) {
-      int e = i * 32 + lane;
-      v[i] = e < experts ? row[e] : -INFINITY;
-      mx = fmaxf(mx, v[i]);
-    }
+  for (int i = 0; i < kPerLane; ++i) {
+    const int e = i * 32 + lane;
+    key[i] = e < experts ? logit_key(__ldg(row + e)) : 0u;
   }
+  uint32_t best;
+  int best_e;
+  auto rescan = [&]() {  // lowest index first on ties (i ascending, strict >)
+    best = 0u;
+    best_e = 0x7fffffff;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int i = 0; i < kPerLane; ++i)
+      if (key[i] > best) { best = key[i]; best_e = i * 32 + lane; }
+  };
+  rescan();
 
+  float mx = 0.f;      // the first winner's logit
   float sel_sum = 0.f;
-  float my_w = 0.f;   // lane j keeps the j-th selected expert's exp(logit - max)
+  uint32_t my_key = 0;  // lane j keeps the j-th winner of the current 32
   int my_id = 0;
   for (int j = 0; j < topk; ++j) {
-    // local arg-max (lowest index first on ties: i ascending, strict >)
-    float best = -INFINITY;
-    int best_e = 0x7fffffff;
+    const uint32_t win = __reduce_max_sync(0xffffffffu, best);
+    const int win_e = __reduce_min_sync(0xffffffffu, best == win ? best_e : 0x7fffffff);
+    if (j == 0) mx = key_logit(win);
+    if (lane == (j & 31)) { my_key = win; my_id = win_e; }
+    // retire the winner (as -inf, like an expert masked by the caller)
+    if (best_e == win_e) {
 #pragma unroll
-    for (int i = 0; i < kRouteMaxPerLane; ++i) {
-      if (i < per_lane) {
-        int e = i * 32 + lane;
-        if (e < experts && (v[i] > best || (v[i] == best && e < best_e))) { best = v[i]; best_e = e; }
-      }
+      for (int i = 0; i < kPerLane; ++i)
+        if (i * 32 + lane == win_e) key[i] = kKeyNegInf;
+      rescan();
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
-    // retire the winner
-    if ((best_e & 31) == lane) {
-#pragma unroll
-      for (int i = 0; i < kRouteMaxPerLane; ++i)
-        if (i == (best_e >> 5)) v[i] = -INFINITY;
-    }
-    float p = expf(best - mx);
-    sel_sum += p;
-    if (lane == (j & 31)) { my_w = p; my_id = best_e; }
     if ((j & 31) == 31 || j == topk - 1) {
-      // flush up to 32 selections; the renormalisation needs the final sum, so
-      // weights are written unnormalised here and scaled below when topk > 32
-      int base = j & ~31;
-      if (base + lane <= j) {
+      // up to 32 selections; beyond 32 the sum is not final yet, so the weights are written
+      // unnormalised and scaled below
+      const int base = j & ~31;
+      const int n = j - base + 1;
+      float p = expf(key_logit(my_key) - mx);
+      for (int i = 0; i < n; ++i) sel_sum += __shfl_sync(0xffffffffu, p, i);
+      if (topk <= 32) p *= 1.0f / sel_sum;
+      if (lane < n) {
         ids[size_t(token) * topk + base + lane] = my_id;
-        weights[size_t(token) * topk + base + lane] = my_w;
+        weights[size_t(token) * topk + base + lane] = p;
       }
     }
   }
-  __syncwarp();
-  const float inv = 1.0f / sel_sum;
-  for (int j = lane; j < topk; j += 32) weights[size_t(token) * topk + j] *= inv;
+  if (topk > 32) {
+    __syncwarp();
+    const float inv = 1.0f / sel_sum;
+    for (int j = lane; j < topk; j += 32) weights[size_t(token) * topk + j] *= inv;
+  }
 }
 
 // ---------------------------------------------------------------- align
@@ -331,14 +347,23 @@ align_fused_kernel(const int* __restrict__ topk_ids, const int* __restrict__ exp
 
 int launch_route_topk(const float* logits, int tokens, int experts, int topk, int* ids,
                       float* weights, cudaStream_t stream) {
-  MB200_REQUIRE(experts >= 1 && experts <= 32 * kRouteMaxPerLane, kUnsupportedShape,
-                "route_topk: %d experts, supported 1..%d", experts, 32 * kRouteMaxPerLane);
+  MB200_REQUIRE(experts >= 1 && experts <= kRouteMaxExperts, kUnsupportedShape,
+                "route_topk: %d experts, supported 1..%d", experts, kRouteMaxExperts);
   MB200_REQUIRE(topk >= 1 && topk <= experts, kInvalidArgument, "route_topk: topk=%d with %d experts",
                 topk, experts);
   if (tokens == 0) return kOk;
   const int warps = 4;
-  route_topk_kernel<<<(tokens + warps - 1) / warps, warps * 32, 0, stream>>>(logits, tokens, experts,
-                                                                              topk, ids, weights);
+  const int blocks = (tokens + warps - 1) / warps;
+  const int per_lane = (experts + 31) / 32;
+  auto launch = [&](auto kernel) {
+    kernel<<<blocks, warps * 32, 0, stream>>>(logits, tokens, experts, topk, ids, weights);
+  };
+  if (per_lane <= 1) launch(route_topk_kernel<1>);
+  else if (per_lane <= 2) launch(route_topk_kernel<2>);
+  else if (per_lane <= 4) launch(route_topk_kernel<4>);
+  else if (per_lane <= 8) launch(route_topk_kernel<8>);
+  else if (per_lane <= 16) launch(route_topk_kernel<16>);
+  else launch(route_topk_kernel<32>);
   MB200_CHECK_CUDA(cudaGetLastError());
   return kOk;
 }

@@ -29,6 +29,7 @@
 // chunks of parity (w-2)/4, at most 64 columns x 2 accumulators per thread.
 
 #include <atomic>
+#include <type_traits>
 
 #include "layer.cuh"
 
@@ -402,25 +403,28 @@ grouped_gemm_fp8_cols_kernel(const __grid_constant__ CUtensorMap map_w,
         if (!ok) break;
         const int feature = tc.fblock * 128 + r;
         uint8_t* out = reinterpret_cast<uint8_t*>(args.out);
+        auto store = [&](auto power_of_two) {
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          if (m < my_chunks) {
-            const int c = cgroup + 2 * m;
+          for (int m = 0; m < 4; ++m) {
+            if (m < my_chunks) {
+              const int c = cgroup + 2 * m;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int col = c * 16 + j;
-              float amax = fmaxf(fmaxf(tail->col_amax[par][0][col], tail->col_amax[par][1][col]),
-                                 fmaxf(tail->col_amax[par][2][col], tail->col_amax[par][3][col]));
-              amax = fmaxf(amax, 1e-10f);
-              const float scale = fp8_group_scale(amax, args.ue8m0);
-              if (col < tc.valid) {
-                const float q = fminf(fmaxf(__fdiv_rn(acc0[m * 16 + j], scale), -448.f), 448.f);
-                if (feature < args.out_cols) out[size_t(tc.row0 + col) * args.out_cols + feature] = to_e4m3(q);
-                if (r == 0) args.out_scale_t[size_t(tc.fblock) * args.row_capacity + tc.row0 + col] = scale;
+              for (int j = 0; j < 16; ++j) {
+                const int col = c * 16 + j;
+                float amax = fmaxf(fmaxf(tail->col_amax[par][0][col], tail->col_amax[par][1][col]),
+                                   fmaxf(tail->col_amax[par][2][col], tail->col_amax[par][3][col]));
+                amax = fmaxf(amax, 1e-10f);
+                const float scale = fp8_group_scale(amax, decltype(power_of_two)::value);
+                if (col < tc.valid) {
+                  const float q = Fp8Divider<decltype(power_of_two)::value>(scale).clamped(acc0[m * 16 + j]);
+                  if (feature < args.out_cols) out[size_t(tc.row0 + col) * args.out_cols + feature] = to_e4m3(q);
+                  if (r == 0) args.out_scale_t[size_t(tc.fblock) * args.row_capacity + tc.row0 + col] = scale;
+                }
               }
             }
           }
-        }
+        };
+        if (args.ue8m0) store(std::true_type{}); else store(std::false_type{});
       } else {
         const int feature = tc.fblock * 256 + r;
         __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(args.out);

@@ -410,11 +410,13 @@ static int moe_forward_16bit(int fp16, const void* hidden_states, const void* w1
   __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(ws + l.act);
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(ws + l.y);
 
+  // the row gather runs inside the gate/up GEMM kernel (dispatch warps); the sort resets its counters
+  sched.clear = reinterpret_cast<int*>(ws + l.granules);
+  sched.clear_ints = l.granule_bytes / 4;
   mark_stage(0, s);
   if ((rc = launch_align(topk_ids, tokens * topk, expert_map, local_experts, sched, cap,
                          reinterpret_cast<int*>(ws + l.scratch), s))) return rc;
   mark_stage(1, s);
-  // the row gather runs inside the gate/up GEMM kernel (dispatch warps); only its counters are reset here
   FusedDispatch disp{};
   disp.src.ptr[0] = const_cast<void*>(hidden_states);
   disp.rank = 0;
@@ -423,10 +425,9 @@ static int moe_forward_16bit(int fp16, const void* hidden_states, const void* w1
   disp.topk = topk;
   disp.vec_per_row = hidden / 8;
   disp.rows_out = reinterpret_cast<uint4*>(xg);
-  disp.granule_done = reinterpret_cast<int*>(ws + l.granules);
+  disp.granule_done = sched.clear;
   disp.granule_target = kDispatchWarpsPerCta;
   disp.enabled = kDispatchFused;
-  MB200_CHECK_CUDA(cudaMemsetAsync(disp.granule_done, 0, size_t(l.granule_bytes), s));
   mark_stage(2, s);
   if ((rc = run_gemm_stage(kGateUpSwiglu, xg, cap, w1, local_experts, hidden, intermediate, sched.counts,
                            sched.mtile_prefix, sched.sorted_ids, nullptr, act, status, device, s,
@@ -529,6 +530,10 @@ int mb200_moe_forward_fp8(const void* hidden_states, const void* w1, const void*
   float* acts_t = reinterpret_cast<float*>(ws + l.acts);
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(ws + l.y);
 
+  if (pad == kTileM) {  // arrival counters of the fused gather, reset by the sort
+    sched.clear = reinterpret_cast<int*>(ws + l.granules);
+    sched.clear_ints = l.granule_bytes / 4;
+  }
   mark_stage(0, s);
   if ((rc = launch_align(topk_ids, tokens * topk, expert_map, local_experts, sched, cap,
                          reinterpret_cast<int*>(ws + l.scratch), s))) return rc;
@@ -544,8 +549,7 @@ int mb200_moe_forward_fp8(const void* hidden_states, const void* w1, const void*
   self_s.ptr[0] = xs_tok;
   FusedDispatchFp8 disp{};
   if (pad == kTileM) {
-    // 128-row-tile kernel: the gather runs inside the gate/up GEMM kernel (helper warps); only its
-    // counters are reset here
+    // 128-row-tile kernel: the gather runs inside the gate/up GEMM kernel (helper warps)
     disp.xq = self_q;
     disp.xs = self_s;
     disp.rank = 0;
@@ -555,9 +559,8 @@ int mb200_moe_forward_fp8(const void* hidden_states, const void* w1, const void*
     disp.groups_per_row = hidden / 128;
     disp.rows_out = reinterpret_cast<uint4*>(xq);
     disp.scales_t_out = xs_t;
-    disp.granule_done = reinterpret_cast<int*>(ws + l.granules);
+    disp.granule_done = sched.clear;
     disp.enabled = 1;
-    MB200_CHECK_CUDA(cudaMemsetAsync(disp.granule_done, 0, size_t(l.granule_bytes), s));
   } else if ((rc = launch_gather_rows_peer_fp8(self_q, self_s, 0, 1, int(tokens), topk, sched, local_experts, hidden,
                                                xq, xs_t, cap, s))) {
     return rc;

@@ -170,9 +170,6 @@ int mb200_dist_forward(int precision, int expert_parallel, const void* hidden_st
   if ((rc = launch_gather_routing(offset_table(symmetric_ptrs, world, sl.ids),
                                   offset_table(symmetric_ptrs, world, sl.weights), rank, world,
                                   int(tokens * topk), ids_all, weights_all, s))) return rc;
-  if ((rc = launch_align(ids_all, all_tokens * topk, expert_parallel ? expert_map : nullptr, local_experts, sched,
-                         cap, reinterpret_cast<int*>(ws + l.scratch), s))) return rc;
-  mark_stage(1, s);
   // Which fused forms apply: the 16-bit kernels and the fp8 128-row-tile kernel have dispatch and
   // push warps; the fp8 tokens-on-columns kernel (few rows per expert) keeps separate stages.
   const bool fp8_rows = fp8 && pad == kTileM;
@@ -180,7 +177,13 @@ int mb200_dist_forward(int precision, int expert_parallel, const void* hidden_st
   const bool push_combine = expert_parallel && fused_kernels;
   int* granule_done = reinterpret_cast<int*>(ws + l.granules);
   int* block_done = reinterpret_cast<int*>(ws + l.blocks);
-  if (fused_kernels) MB200_CHECK_CUDA(cudaMemsetAsync(granule_done, 0, size_t(l.counter_span), s));
+  if (fused_kernels) {  // both counter arrays (adjacent) are reset by the sort
+    sched.clear = granule_done;
+    sched.clear_ints = l.counter_span / 4;
+  }
+  if ((rc = launch_align(ids_all, all_tokens * topk, expert_parallel ? expert_map : nullptr, local_experts, sched,
+                         cap, reinterpret_cast<int*>(ws + l.scratch), s))) return rc;
+  mark_stage(1, s);
   FusedDispatch disp{};       // 16-bit: the dispatch pulls run inside the gate/up GEMM kernel
   FusedDispatchFp8 disp8{};   // fp8, 128-row tiles: likewise (e4m3 rows + scales)
   const PeerTable payload = offset_table(symmetric_ptrs, world, sl.payload);

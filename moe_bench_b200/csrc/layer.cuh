@@ -27,6 +27,8 @@ struct Schedule {
   int* sorted_ids;    // [P]    flat assignment index (token*k + kpos) per row, -1 = padding
   int* inverse;       // [A]    row of each assignment, -1 = expert not on this rank
   int pad_rows;       //        granule every expert segment is padded to
+  int* clear = nullptr;    // counters the sort sets to zero on its way (the GEMMs' arrival counters)
+  int64_t clear_ints = 0;
 };
 
 // ---- route_align.cu ---------------------------------------------------------------

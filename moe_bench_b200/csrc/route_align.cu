@@ -11,10 +11,10 @@
 //    reproduces the slot order of the reference's schedule builder on one rank
 //    (tk_scheme.py:98-126, equal to the argsort key of tk_scheme.py:338-342)
 //    and replaces the moe_align_block_size step inside fused_experts
-//    (baseline.py:67).  Work is cut into contiguous "units" of assignments, one
-//    warp each: per-unit warp-shuffle histograms (match.any), an exclusive scan
-//    over units and experts, then a scatter that replays the same match.any
-//    ranks, so the order inside an expert is ascending n whatever the grid.
+//    (baseline.py:67).  Work is cut into contiguous chunks of assignments, one
+//    warp each: per-warp histograms (match.any), exclusive scans over warps,
+//    blocks and experts, then a scatter that replays the same match.any ranks,
+//    so the order inside an expert is ascending n whatever the grid.
 
 #include "layer.cuh"
 
@@ -109,238 +109,224 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, 
 }
 
 // ---------------------------------------------------------------- align
-constexpr int kAlignWarps = 8;
-constexpr int kAlignThreads = kAlignWarps * 32;
-constexpr int kMaxUnits = 1024;
-constexpr int kFusedMaxAssignments = 8192;  // beyond this the three-kernel form is faster (about 35 us flat)
-constexpr int kFusedWarps = 32;
+// The flat assignments are cut into chunks, one per warp, and the warps into blocks.  At most two
+// launches: `align_count_kernel` writes one histogram per block, `align_scatter_kernel` sums the
+// histograms of the blocks before its own, scans the experts and places its assignments, every
+// block redoing the (small) scans for itself, so no single-block pass sits between the two.  One
+// block needs no histogram but its own: up to kOneBlockAssignments a single launch does it all.
+// The work is latency, not bandwidth (8192 tokens x top-8: 0.8 MB): chunks are short, so that many
+// warps wait at the same time, and everything a block shares stays in shared memory.  Measured
+// between stage events (launch gaps included): 8192 tokens, 256 experts 44 -> 32 us; 32768 tokens,
+// 32 local experts 31 -> 21 us; against count, one-block scan and scatter as three kernels, with the
+// arrival counters of the GEMMs cleared by a memset of their own.
+constexpr int kMaxUnits = 1024;            // scratch: this many ints per expert
+constexpr int kMaxAlignWarps = 32;
+constexpr int kMinChunk = 64;              // assignments per warp
+constexpr int kOneBlockAssignments = 4096;
 
-__host__ __device__ inline int64_t unit_chunk(int64_t assignments, int units_cap) {
-  int64_t chunk = (assignments + units_cap - 1) / units_cap;
+struct AlignShape {
+  int warps;   // per block: the per-warp counters of a block fit 48 KiB of shared memory
+  int blocks;
+  int64_t chunk;
+};
+AlignShape align_shape(int64_t assignments, int experts) {
+  AlignShape s;
+  s.warps = experts <= 256 ? kMaxAlignWarps : 8;
+  const int64_t max_blocks = assignments <= kOneBlockAssignments && s.warps == kMaxAlignWarps ? 1 : kMaxUnits / 4;
+  int64_t chunk = (assignments + max_blocks * s.warps - 1) / (max_blocks * s.warps);
   chunk = (chunk + 31) / 32 * 32;
-  // a warp walks its unit 32 assignments at a time, one dependent load per step: short units
-  // (more warps in flight) keep the walk from being a chain of load latencies
-  return chunk < 256 ? 256 : chunk;
+  s.chunk = chunk < kMinChunk ? kMinChunk : chunk;
+  const int64_t per_block = s.chunk * s.warps;
+  s.blocks = assignments <= per_block ? 1 : int((assignments + per_block - 1) / per_block);
+  return s;
 }
 
 __device__ __forceinline__ int slot_of(const int* topk_ids, const int* expert_map, int64_t n,
-                                       int64_t assignments, int local_experts) {
-  if (n >= assignments) return -1;
+                                       int local_experts) {
   int e = __ldg(topk_ids + n);
   if (expert_map) e = (e >= 0) ? __ldg(expert_map + e) : -1;
   return (e >= 0 && e < local_experts) ? e : -1;
 }
 
-// Walk one unit in order, 32 assignments at a time.  `running[e]` counts the
-// unit's assignments to expert e seen so far.  Emit(n, slot, rank) gets the rank
-// of assignment n among the unit's assignments to the same expert.
+// Walk one chunk in order, 32 assignments at a time (the loads of four steps in flight
+// together).  Emit(n, slot, before, peers): `peers` are the lanes with the same slot, `before`
+// how many of them come first; called by every lane whose assignment exists.
 template <class Emit>
-__device__ __forceinline__ void walk_unit(const int* topk_ids, const int* expert_map,
-                                          int64_t begin, int64_t end, int64_t assignments,
-                                          int local_experts, int* running, Emit emit) {
+__device__ __forceinline__ void walk_chunk(const int* topk_ids, const int* expert_map, int64_t begin,
+                                           int64_t end, int local_experts, Emit emit) {
+  constexpr int kSteps = 4;
   const int lane = threadIdx.x & 31;
-  for (int64_t base = begin; base < end; base += 32) {
-    const int64_t n = base + lane;
-    const int slot = (n < end) ? slot_of(topk_ids, expert_map, n, assignments, local_experts) : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, slot);
-    if (slot >= 0) {
-      const int before = __popc(peers & ((1u << lane) - 1u));
-      const int seen = running[slot];
-      emit(n, slot, seen + before);
-    } else if (n < assignments && n < end) {
-      emit(n, -1, 0);
+  for (int64_t base = begin; base < end; base += 32 * kSteps) {
+    int slot[kSteps];
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+      const int64_t n = base + 32 * i + lane;
+      slot[i] = n < end ? slot_of(topk_ids, expert_map, n, local_experts) : -1;
     }
-    __syncwarp();
-    if (slot >= 0 && (peers & ((1u << lane) - 1u)) == 0) running[slot] += __popc(peers);
-    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+      if (base + 32 * i >= end) break;
+      const int64_t n = base + 32 * i + lane;
+      const unsigned peers = __match_any_sync(0xffffffffu, slot[i]);
+      if (n < end) emit(n, slot[i], __popc(peers & ((1u << lane) - 1u)), peers);
+      __syncwarp();
+    }
   }
 }
 
 __global__ void align_count_kernel(const int* __restrict__ topk_ids, const int* __restrict__ expert_map,
-                                   int64_t assignments, int local_experts, int64_t chunk, int units,
-                                   int* __restrict__ unit_hist) {
-  extern __shared__ int hist_smem[];
-  const int warp = threadIdx.x >> 5;
-  const int unit = blockIdx.x * kAlignWarps + warp;
-  int* running = hist_smem + warp * local_experts;
-  for (int e = threadIdx.x & 31; e < local_experts; e += 32) running[e] = 0;
-  __syncwarp();
-  if (unit >= units) return;
-  const int64_t begin = int64_t(unit) * chunk;
+                                   int64_t assignments, int local_experts, int64_t chunk,
+                                   int* __restrict__ block_hist) {
+  extern __shared__ int hist[];  // [E]
+  for (int e = threadIdx.x; e < local_experts; e += blockDim.x) hist[e] = 0;
+  __syncthreads();
+  const int64_t unit = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t begin = unit * chunk < assignments ? unit * chunk : assignments;
   const int64_t end = begin + chunk < assignments ? begin + chunk : assignments;
-  walk_unit(topk_ids, expert_map, begin, end, assignments, local_experts, running,
-            [](int64_t, int, int) {});
-  for (int e = threadIdx.x & 31; e < local_experts; e += 32)
-    unit_hist[size_t(unit) * local_experts + e] = running[e];
+  walk_chunk(topk_ids, expert_map, begin, end, local_experts, [&](int64_t, int slot, int before, unsigned peers) {
+    if (slot >= 0 && before == 0) atomicAdd(hist + slot, __popc(peers));
+  });
+  __syncthreads();
+  for (int e = threadIdx.x; e < local_experts; e += blockDim.x)
+    block_hist[size_t(blockIdx.x) * local_experts + e] = hist[e];
 }
 
-// One block.  unit_hist[u][e] becomes the exclusive prefix over units; counts and
-// the cumulative M-tile table are written.  The block's threads form up to 32 groups
-// of E threads (thread = one expert, consecutive threads = consecutive experts, so
-// every load is a coalesced row segment); each group scans a contiguous range of
-// units in two passes: range sums into `part` ([groups][E] ints of shared memory,
-// at most blockDim.x), then the prefix starting from the sums of the groups before it.
-constexpr int kScanMaxGroups = 32;
-
-__device__ void scan_units_and_experts(int* unit_hist, int units, int local_experts, int* counts,
-                                       int* mtile_prefix, int* smem_tiles /*[E+1]*/, int* part, int pad) {
+// Shared memory, ints: per_warp [warps][E] | total [E] | base [E] | prefix [E+1] | part [2][threads]
+__global__ void __launch_bounds__(kMaxAlignWarps * 32)
+align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ expert_map, int64_t assignments,
+                     int local_experts, int64_t chunk, const int* __restrict__ block_hist,
+                     int* __restrict__ counts, int* __restrict__ mtile_prefix, int* __restrict__ sorted_ids,
+                     int* __restrict__ inverse, int64_t row_capacity, int pad, int* __restrict__ clear,
+                     int64_t clear_ints) {
+  extern __shared__ int smem[];
   const int E = local_experts;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* per_warp = smem;
+  int* total = per_warp + warps * E;
+  int* base = total + E;
+  int* prefix = base + E;
+  int* part = prefix + E + 1;
+  const int nb = gridDim.x;
+
+  // counters of the kernels that follow (arrivals per granule / token block)
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < clear_ints; i += int64_t(nb) * blockDim.x)
+    clear[i] = 0;
+
+  // 1. this block's assignments per (warp, expert)
+  const int64_t unit = int64_t(blockIdx.x) * warps + warp;
+  const int64_t begin = unit * chunk < assignments ? unit * chunk : assignments;
+  const int64_t end = begin + chunk < assignments ? begin + chunk : assignments;
+  int* running = per_warp + warp * E;
+  for (int e = lane; e < E; e += 32) running[e] = 0;
+  __syncwarp();
+  walk_chunk(topk_ids, expert_map, begin, end, E, [&](int64_t, int slot, int before, unsigned peers) {
+    if (slot >= 0 && before == 0) running[slot] += __popc(peers);
+  });
+  __syncthreads();
+
+  // 2. total[e] over all blocks, base[e] over the blocks before this one.  Thread groups of E
+  // threads take every groups-th row of the histogram (or of per_warp when there is one block).
+  const int rows = nb > 1 ? nb : warps;
+  constexpr int kMaxGroups = 32;
   int groups = E < int(blockDim.x) ? int(blockDim.x) / E : 1;
-  if (groups > kScanMaxGroups) groups = kScanMaxGroups;
-  const int per_group = (units + groups - 1) / groups;
-  for (int e0 = 0; e0 < E; e0 += blockDim.x) {  // one trip unless E exceeds the block
+  if (groups > kMaxGroups) groups = kMaxGroups;
+  for (int e0 = 0; e0 < E; e0 += blockDim.x) {
     const int g = groups > 1 ? int(threadIdx.x) / E : 0;
     const int e = e0 + (groups > 1 ? int(threadIdx.x) % E : int(threadIdx.x));
-    const bool active = e < E && g < groups;
-    const int u_lo = g * per_group < units ? g * per_group : units;
-    const int u_hi = u_lo + per_group < units ? u_lo + per_group : units;
-    int run = 0;
-    if (groups > 1) {
-      if (active) {
-        int sum = 0;
-        for (int u0 = u_lo; u0 < u_hi; u0 += 8) {
-          int v[8];  // loads first, so eight of them are in flight together
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            v[i] = (u0 + i < u_hi) ? unit_hist[size_t(u0 + i) * E + e] : 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) sum += v[i];
-        }
-        part[g * E + e] = sum;
-      }
-      __syncthreads();
-      if (active)
-        for (int w = 0; w < g; ++w) run += part[w * E + e];
-    }
-    if (active) {
-      for (int u0 = u_lo; u0 < u_hi; u0 += 8) {
-        int v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          v[i] = (u0 + i < u_hi) ? unit_hist[size_t(u0 + i) * E + e] : 0;
+    if (e < E && g < groups) {
+      int all = 0, prev = 0;
+      for (int r0 = g; r0 < rows; r0 += 8 * groups) {
+        int v[8];  // loads first, so eight of them are in flight together
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          if (u0 + i < u_hi) unit_hist[size_t(u0 + i) * E + e] = run;
-          run += v[i];
+          const int r = r0 + i * groups;
+          v[i] = r >= rows ? 0 : nb > 1 ? __ldg(block_hist + size_t(r) * E + e) : per_warp[r * E + e];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          all += v[i];
+          if (nb > 1 && r0 + i * groups < int(blockIdx.x)) prev += v[i];
         }
       }
-      if (g == groups - 1) {  // the last group's running sum is the expert's total
-        counts[e] = run;
-        smem_tiles[e] = (run + pad - 1) / pad;
+      if (groups == 1) {
+        total[e] = all;
+        base[e] = prev;
+      } else {
+        part[g * E + e] = all;
+        part[blockDim.x + g * E + e] = prev;
       }
     }
-    if (groups > 1) __syncthreads();  // `part` is reused by the next trip
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    // warp scan: each lane owns a contiguous run of experts
-    const int lane = threadIdx.x;
-    const int per = (local_experts + 31) / 32;
-    const int lo = lane * per;
-    const int hi = lo + per < local_experts ? lo + per : local_experts;
+  if (groups > 1) {
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+      int all = 0, prev = 0;
+      for (int g = 0; g < groups; ++g) {
+        all += part[g * E + e];
+        prev += part[blockDim.x + g * E + e];
+      }
+      total[e] = all;
+      base[e] = prev;
+    }
+    __syncthreads();
+  }
+
+  // 3. cumulative row blocks per expert: each lane of warp 0 owns a run of experts
+  if (warp == 0) {
+    const int per = (E + 31) / 32;
+    const int lo = lane * per < E ? lane * per : E;
+    const int hi = lo + per < E ? lo + per : E;
     int sum = 0;
-    for (int e = lo; e < hi; ++e) sum += smem_tiles[e];
+    for (int e = lo; e < hi; ++e) sum += (total[e] + pad - 1) / pad;
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      int t = __shfl_up_sync(0xffffffffu, incl, o);
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
     int run = incl - sum;
     for (int e = lo; e < hi; ++e) {
-      int t = smem_tiles[e];
-      mtile_prefix[e] = run;
-      run += t;
+      prefix[e] = run;
+      run += (total[e] + pad - 1) / pad;
     }
-    if (lane == 31) mtile_prefix[local_experts] = incl;
+    if (lane == 31) prefix[E] = incl;
   }
-}
-
-__global__ void align_scan_kernel(int* unit_hist, int units, int local_experts, int* counts,
-                                  int* mtile_prefix, int pad) {
-  extern __shared__ int tiles_smem[];  // [E+1] tiles per expert, then [blockDim.x] partial sums
-  scan_units_and_experts(unit_hist, units, local_experts, counts, mtile_prefix, tiles_smem,
-                         tiles_smem + (local_experts + 1), pad);
-}
-
-// Mark the padding rows of expert e with -1; `lane`/`width` are the caller's
-// position in the group of threads that shares the expert.
-__device__ __forceinline__ void fill_padding(const int* counts, const int* mtile_prefix, int e,
-                                             int* sorted_ids, int64_t row_capacity, int lane, int width,
-                                             int pad) {
-  const int64_t begin = int64_t(mtile_prefix[e]) * pad + counts[e];
-  int64_t end = int64_t(mtile_prefix[e + 1]) * pad;
-  if (end > row_capacity) end = row_capacity;
-  for (int64_t p = begin + lane; p < end; p += width) sorted_ids[p] = -1;
-}
-
-__global__ void align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ expert_map,
-                                     int64_t assignments, int local_experts, int64_t chunk, int units,
-                                     const int* __restrict__ unit_base, const int* __restrict__ counts,
-                                     const int* __restrict__ mtile_prefix, int* __restrict__ sorted_ids,
-                                     int* __restrict__ inverse, int64_t row_capacity, int pad) {
-  extern __shared__ int hist_smem[];
-  // one warp per expert, experts strided over every warp of the grid
-  for (int e = blockIdx.x * kAlignWarps + (threadIdx.x >> 5); e < local_experts; e += gridDim.x * kAlignWarps)
-    fill_padding(counts, mtile_prefix, e, sorted_ids, row_capacity, threadIdx.x & 31, 32, pad);
-
-  const int warp = threadIdx.x >> 5;
-  const int unit = blockIdx.x * kAlignWarps + warp;
-  int* running = hist_smem + warp * local_experts;
-  for (int e = threadIdx.x & 31; e < local_experts; e += 32) running[e] = 0;
-  __syncwarp();
-  if (unit >= units) return;
-  const int64_t begin = int64_t(unit) * chunk;
-  const int64_t end = begin + chunk < assignments ? begin + chunk : assignments;
-  const int* base = unit_base + size_t(unit) * local_experts;
-  walk_unit(topk_ids, expert_map, begin, end, assignments, local_experts, running,
-            [&](int64_t n, int slot, int rank) {
-              if (slot < 0) { inverse[n] = -1; return; }
-              const int64_t row = int64_t(mtile_prefix[slot]) * pad + base[slot] + rank;
-              if (row < row_capacity) sorted_ids[row] = int(n);
-              inverse[n] = int(row);
-            });
-}
-
-// Whole step in one block of 32 warps (small problems: one launch instead of three).
-__global__ void __launch_bounds__(kFusedWarps * 32)
-align_fused_kernel(const int* __restrict__ topk_ids, const int* __restrict__ expert_map,
-                   int64_t assignments, int local_experts, int* __restrict__ counts,
-                   int* __restrict__ mtile_prefix, int* __restrict__ sorted_ids,
-                   int* __restrict__ inverse, int64_t row_capacity, int* __restrict__ unit_hist, int pad) {
-  extern __shared__ int smem[];
-  int* tiles_smem = smem;                              // [E+1]
-  int* running_all = smem + (local_experts + 1);       // [32][E]
-  const int warp = threadIdx.x >> 5;
-  int64_t chunk = (assignments + kFusedWarps - 1) / kFusedWarps;
-  chunk = (chunk + 31) / 32 * 32;
-  const int64_t begin = warp * chunk < assignments ? warp * chunk : assignments;
-  const int64_t end = begin + chunk < assignments ? begin + chunk : assignments;
-  int* running = running_all + warp * local_experts;
-
-  for (int e = threadIdx.x & 31; e < local_experts; e += 32) running[e] = 0;
-  __syncwarp();
-  walk_unit(topk_ids, expert_map, begin, end, assignments, local_experts, running,
-            [](int64_t, int, int) {});
-  for (int e = threadIdx.x & 31; e < local_experts; e += 32)
-    unit_hist[size_t(warp) * local_experts + e] = running[e];
   __syncthreads();
-  // the per-warp counters are free between the two walks and serve as the scan's partial sums
-  scan_units_and_experts(unit_hist, kFusedWarps, local_experts, counts, mtile_prefix, tiles_smem,
-                         running_all, pad);
+
+  // 4. first row of every (warp, expert): expert's first row + blocks before + warps before
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = prefix[e] * pad + base[e];
+    for (int w0 = 0; w0 < warps; w0 += 8) {  // 8 or 32 warps
+      int v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = per_warp[(w0 + i) * E + e];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        per_warp[(w0 + i) * E + e] = run;
+        run += v[i];
+      }
+    }
+  }
+  if (blockIdx.x == 0) {
+    for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = total[e];
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) mtile_prefix[e] = prefix[e];
+  }
   __syncthreads();
-  for (int e = warp; e < local_experts; e += kFusedWarps)
-    fill_padding(counts, mtile_prefix, e, sorted_ids, row_capacity, threadIdx.x & 31, 32, pad);
-  for (int e = threadIdx.x & 31; e < local_experts; e += 32) running[e] = 0;
-  __syncwarp();
-  const int* base = unit_hist + size_t(warp) * local_experts;
-  walk_unit(topk_ids, expert_map, begin, end, assignments, local_experts, running,
-            [&](int64_t n, int slot, int rank) {
-              if (slot < 0) { inverse[n] = -1; return; }
-              const int64_t row = int64_t(mtile_prefix[slot]) * pad + base[slot] + rank;
-              if (row < row_capacity) sorted_ids[row] = int(n);
-              inverse[n] = int(row);
-            });
+
+  // 5. place this warp's assignments; the experts' padding rows are shared out over all warps
+  walk_chunk(topk_ids, expert_map, begin, end, E, [&](int64_t n, int slot, int before, unsigned peers) {
+    if (slot < 0) { inverse[n] = -1; return; }
+    const int row = running[slot] + before;
+    if (row < row_capacity) sorted_ids[row] = int(n);
+    inverse[n] = row;
+    __syncwarp(peers);  // the peers have read the counter
+    if (before == 0) running[slot] += __popc(peers);
+  });
+  for (int e = blockIdx.x * warps + warp; e < E; e += nb * warps) {
+    int64_t stop = int64_t(prefix[e + 1]) * pad;
+    if (stop > row_capacity) stop = row_capacity;
+    for (int64_t p = int64_t(prefix[e]) * pad + total[e] + lane; p < stop; p += 32) sorted_ids[p] = -1;
+  }
 }
 
 }  // namespace
@@ -382,30 +368,17 @@ int launch_align(const int* topk_ids, int64_t assignments, const int* expert_map
                 "align: %lld assignments do not fit 32-bit row indices", (long long)assignments);
   const int pad = sched.pad_rows;
   MB200_REQUIRE(pad >= 1 && pad <= 1024, kInvalidArgument, "align: pad_rows=%d (1..1024)", pad);
-  const size_t fused_smem = size_t(local_experts + 1 + kFusedWarps * local_experts) * sizeof(int);
-  if (assignments <= kFusedMaxAssignments && fused_smem <= 48 * 1024) {
-    align_fused_kernel<<<1, kFusedWarps * 32, fused_smem, stream>>>(
-        topk_ids, expert_map, assignments, local_experts, sched.counts, sched.mtile_prefix,
-        sched.sorted_ids, sched.inverse, row_capacity, scratch, pad);
-    MB200_CHECK_CUDA(cudaGetLastError());
-    return kOk;
-  }
-  const int64_t chunk = unit_chunk(assignments, kMaxUnits);
-  const int units = int((assignments + chunk - 1) / chunk);
-  const int blocks = (units + kAlignWarps - 1) / kAlignWarps;
-  const size_t hist_smem = size_t(kAlignWarps) * local_experts * sizeof(int);
-  if (blocks > 0) {
-    align_count_kernel<<<blocks, kAlignThreads, hist_smem, stream>>>(
-        topk_ids, expert_map, assignments, local_experts, chunk, units, scratch);
+  const AlignShape sh = align_shape(assignments, local_experts);
+  const int threads = sh.warps * 32;
+  if (sh.blocks > 1) {
+    align_count_kernel<<<sh.blocks, threads, size_t(local_experts) * sizeof(int), stream>>>(
+        topk_ids, expert_map, assignments, local_experts, sh.chunk, scratch);
     MB200_CHECK_CUDA(cudaGetLastError());
   }
-  align_scan_kernel<<<1, 1024, size_t(local_experts + 1 + 1024) * sizeof(int), stream>>>(
-      scratch, units, local_experts, sched.counts, sched.mtile_prefix, pad);
-  MB200_CHECK_CUDA(cudaGetLastError());
-  const int sblocks = blocks > 0 ? blocks : 1;
-  align_scatter_kernel<<<sblocks, kAlignThreads, hist_smem, stream>>>(
-      topk_ids, expert_map, assignments, local_experts, chunk, units, scratch, sched.counts,
-      sched.mtile_prefix, sched.sorted_ids, sched.inverse, row_capacity, pad);
+  const size_t smem = size_t(sh.warps * local_experts + 3 * local_experts + 1 + 2 * threads) * sizeof(int);
+  align_scatter_kernel<<<sh.blocks, threads, smem, stream>>>(
+      topk_ids, expert_map, assignments, local_experts, sh.chunk, scratch, sched.counts, sched.mtile_prefix,
+      sched.sorted_ids, sched.inverse, row_capacity, pad, sched.clear, sched.clear_ints);
   MB200_CHECK_CUDA(cudaGetLastError());
   return kOk;
 }

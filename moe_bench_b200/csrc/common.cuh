@@ -184,6 +184,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, WaitCtx
   const bool ok = mbar_wait_lane(bar, parity, ctx, where);
   return __all_sync(0xffffffffu, ok);
 }
+// One poll, no waiting; the same answer in all lanes.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
+}
 __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, WaitCtx& ctx, int where) {
   uint32_t spins = 0;
   WaitClock clock;
@@ -316,6 +330,29 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
+}
+// 16 lanes x 16 consecutive fp32 columns in the fragment layout of 8x8 matrices: thread i holds,
+// of lane i/4, columns 2*(i%4), +1 in r[0..1] and the same + 8 in r[4..5]; of lane i/4 + 8 in
+// r[2..3] and r[6..7].
+__device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr));
+}
+// Four 8x8 16-bit matrices, transposed, to shared memory: lane i gives the address of row i%8 of matrix i/8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ uint32_t pack_h16x2(float lo, float hi, int fp16) {
+  if (fp16) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");

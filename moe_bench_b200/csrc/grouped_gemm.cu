@@ -70,13 +70,13 @@ struct SmemTail {
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
   uint64_t acc_full[2];
-  uint64_t acc_empty[2];
+  uint64_t acc_empty[2][2];         // [buffer][half]; the gate/up GEMM releases both halves through the first
   uint64_t epi_bar;
   uint32_t tmem_base;
   int abort_flag;
   int max_blocks16;                 // largest expert segment, in 16-row blocks
   int tile_assign[2][kMaxTokens];   // down GEMM: flat assignment of each token column
-  float tile_weight[2][kMaxTokens];
+  alignas(8) float tile_weight[2][kMaxTokens];
   int prefix[kMaxExperts + 1];      // cumulative 16-row blocks per expert
   int tb_prefix[kMaxExperts + 1];   // cumulative token blocks per expert
 };
@@ -118,22 +118,24 @@ struct TileCoord {
 
 // Tiles are numbered expert-major; inside an expert the token blocks of one
 // feature block are adjacent, so CTAs running side by side stream the same
-// weight rows and all but the first read hit L2.
+// weight rows and all but the first read hit L2.  Called by whole warps (E <= 1024).
 __device__ __forceinline__ TileCoord decode_tile(int tile, const SmemTail* t, const int* counts,
                                                  int num_experts, int n_fblocks, int tb_rows) {
-  int lo = 0, hi = num_experts;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (t->tb_prefix[mid] * n_fblocks <= tile) lo = mid; else hi = mid - 1;
-  }
+  // the last expert whose first tile is not past `tile`: 32 coarse probes, then one per expert
+  const int lane = threadIdx.x & 31;
+  const int step = (num_experts + 31) / 32;
+  const int coarse = lane * step;
+  int lo = (__popc(__ballot_sync(0xffffffffu, coarse < num_experts && t->tb_prefix[coarse] * n_fblocks <= tile)) - 1) * step;
+  const int fine = lo + lane;
+  lo += __popc(__ballot_sync(0xffffffffu, lane < step && fine < num_experts && t->tb_prefix[fine] * n_fblocks <= tile)) - 1;
   TileCoord c;
   c.expert = lo;
   const int local = tile - t->tb_prefix[lo] * n_fblocks;
   const int nb = t->tb_prefix[lo + 1] - t->tb_prefix[lo];
-  c.fblock = local / nb;
+  c.fblock = nb == 1 ? local : local / nb;
   const int j = local - c.fblock * nb;
   const int blocks16 = t->prefix[lo + 1] - t->prefix[lo];
-  const int per = (blocks16 + nb - 1) / nb;  // balanced split of the segment
+  const int per = nb == 1 ? blocks16 : (blocks16 + nb - 1) / nb;  // balanced split of the segment
   const int start16 = j * per;
   int len16 = blocks16 - start16;
   if (len16 > per) len16 = per;
@@ -190,7 +192,8 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&tail->acc_full[b]), 1);
-      mbar_init(smem_u32(&tail->acc_empty[b]), kEpiWarps);
+      mbar_init(smem_u32(&tail->acc_empty[b][0]), kEpiWarps);
+      mbar_init(smem_u32(&tail->acc_empty[b][1]), kEpiWarps);
     }
     mbar_init(smem_u32(&tail->epi_bar), kEpiWarps);
     tail->abort_flag = 0;
@@ -330,28 +333,63 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
       const TileCoord tc = decode_tile(tile, tail, args.counts, E, n_fgroups, geo.tb_rows);
       const uint32_t buf = geo.acc_bufs == 2 ? (it & 1) : 0;
       const uint32_t use = geo.acc_bufs == 2 ? (it >> 1) : it;
-      ok = mbar_wait(smem_u32(&tail->acc_empty[buf]), (use & 1) ^ 1, ctx, 2);
+      const uint32_t free_parity = (use & 1) ^ 1;
+      ok = mbar_wait(smem_u32(&tail->acc_empty[buf][0]), free_parity, ctx, 2);
       if (!ok) break;
       tc_fence_after();
       const uint32_t d0 = tmem_base + buf * 256;
       const uint32_t d1 = d0 + acc1_off;
       const uint32_t fmt = args.fp16 ? 0u : 1u;  // kind::f16 operand format: 0 = f16, 1 = bf16
       const uint32_t idesc = make_idesc(fmt, fmt, 128, uint32_t(tc.ntok));
-      for (int kb = 0; kb < args.k_iters; ++kb) {
+      // one K step into one half: 16 bf16 = 32 bytes of K per instruction, +2 in the 16-byte address field
+      auto multiply = [&](int kb, int from_stage, int half, int k) {
+        const uint32_t w_addr = ring_addr + from_stage * geo.stage_bytes;
+        const uint64_t w_desc = make_kmajor_sw128_desc(w_addr + half * (kWeightBytes / 2));
+        const uint64_t t_desc = make_kmajor_sw128_desc(w_addr + kWeightBytes);
+        umma_bf16(half == 0 ? d0 : d1, w_desc + 2 * k, t_desc + 2 * k, idesc, (kb | k) != 0);
+      };
+      int kb = 0;
+      if (kMode == kDownWeighted) {
+        // The epilogue hands the first half back before the second.  With one accumulator pair the
+        // first K steps (at most as many as the ring holds) go into the first half meanwhile, and
+        // into the second once that is free too.
+        const int ring_steps = geo.stages < args.k_iters ? geo.stages : args.k_iters;
+        int s1 = stage, lead = 0;
+        uint32_t phase1 = phase;
+        for (; geo.acc_bufs == 1 && lead < ring_steps; ++lead) {
+          if (mbar_test(smem_u32(&tail->acc_empty[buf][1]), free_parity)) break;
+          ok = mbar_wait(smem_u32(&tail->full[s1]), phase1, ctx, 3);
+          if (!ok) break;
+          tc_fence_after();
+          if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) multiply(lead, s1, 0, k);
+          }
+          __syncwarp();
+          if (++s1 == geo.stages) { s1 = 0; phase1 ^= 1; }
+        }
+        ok = ok && mbar_wait(smem_u32(&tail->acc_empty[buf][1]), free_parity, ctx, 2);
+        if (!ok) break;
+        tc_fence_after();
+        for (; kb < lead; ++kb) {
+          if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) multiply(kb, stage, 1, k);
+            tc_commit(smem_u32(&tail->empty[stage]));
+          }
+          __syncwarp();
+          if (++stage == geo.stages) { stage = 0; phase ^= 1; }
+        }
+      }
+      for (; kb < args.k_iters; ++kb) {
         ok = mbar_wait(smem_u32(&tail->full[stage]), phase, ctx, 3);
         if (!ok) break;
         tc_fence_after();
         if (lane == 0) {
-          const uint32_t w_addr = ring_addr + stage * geo.stage_bytes;
-          const uint64_t w0_desc = make_kmajor_sw128_desc(w_addr);
-          const uint64_t w1_desc = make_kmajor_sw128_desc(w_addr + kWeightBytes / 2);
-          const uint64_t t_desc = make_kmajor_sw128_desc(w_addr + kWeightBytes);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            // 16 bf16 = 32 bytes of K per instruction: +2 in the 16-byte address field
-            const uint32_t accumulate = (kb | k) != 0;
-            umma_bf16(d0, w0_desc + 2 * k, t_desc + 2 * k, idesc, accumulate);
-            umma_bf16(d1, w1_desc + 2 * k, t_desc + 2 * k, idesc, accumulate);
+            multiply(kb, stage, 0, k);
+            multiply(kb, stage, 1, k);
           }
           // the stage is free once these MMAs have read it
           tc_commit(smem_u32(&tail->empty[stage]));
@@ -471,6 +509,20 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
     uint32_t it = 0;
     uint32_t epi_phase = 0;
     bool ok = true;
+    // Down GEMM: destination row and combine weight of each token column, shared by all feature
+    // rows; thread j looks after column j.  The two loads depend on one another and each waits
+    // behind the weight stream, so the assignment is fetched two tiles ahead and its weight one
+    // tile ahead: with a short K (4 K steps a tile at an intermediate slice of 256) they took as
+    // long as the rest of the tile.
+    static_assert(kMode != kDownWeighted || kEpiWarps * 32 >= kMaxTokens, "one thread per token column");
+    auto fetch_assign = [&](int tile) -> int {
+      if (kMode != kDownWeighted || tile >= total_tiles) return -1;
+      const TileCoord tc = decode_tile(tile, tail, args.counts, E, n_fgroups, geo.tb_rows);
+      return etid < tc.valid ? __ldg(args.sorted_ids + tc.row0 + etid) : -1;
+    };
+    auto fetch_weight = [&](int a) -> float { return kMode == kDownWeighted && a >= 0 ? __ldg(args.row_scale + a) : 0.f; };
+    int assign = fetch_assign(worker), assign_next = fetch_assign(worker + workers);
+    float weight = fetch_weight(assign);
     for (int tile = worker; ok && tile < total_tiles; tile += workers, ++it) {
       const TileCoord tc = decode_tile(tile, tail, args.counts, E, n_fgroups, geo.tb_rows);
       const int fblock = tc.fblock;
@@ -478,19 +530,15 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
       const uint32_t use = geo.acc_bufs == 2 ? (it >> 1) : it;
       const int par = it & 1;
       if (kMode == kDownWeighted) {
-        // per-token destination row and combine weight, shared by all feature rows
-        for (int j = etid; j < tc.ntok; j += kEpiWarps * 32) {
-          int a = -1;
-          float w = 0.f;
-          if (j < tc.valid) {
-            a = __ldg(args.sorted_ids + tc.row0 + j);
-            if (a >= 0) w = __ldg(args.row_scale + a);
-          }
-          tail->tile_assign[par][j] = a;
-          tail->tile_weight[par][j] = w;
+        if (etid < kMaxTokens) {
+          tail->tile_assign[par][etid] = assign;
+          tail->tile_weight[par][etid] = weight;
         }
         ok = epilogue_barrier(&tail->epi_bar, epi_phase, ctx, lane);
         if (!ok) break;
+        assign = assign_next;
+        weight = fetch_weight(assign);
+        assign_next = fetch_assign(tile + 2 * workers);
       }
       ok = mbar_wait(smem_u32(&tail->acc_full[buf]), use & 1, ctx, 4);
       if (!ok) break;
@@ -501,27 +549,55 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
       uint16_t* out_own = kPush ? reinterpret_cast<uint16_t*>(push.dst.ptr[push.rank]) : out;
       const int chunks = tc.ntok >> 4;
 
-      // A thread holds one feature (accumulator row) of 16 tokens; memory wants the
-      // features of a token side by side.  Each 16-token chunk is rounded, transposed
-      // through a 1 KiB per-warp block of shared memory and leaves as 16-byte stores
-      // (8 features of one token per thread), two per thread and output block.
+      // An accumulator row is one feature, memory wants the features of a token side by side.  Each
+      // chunk of 32 features x 16 tokens is read from tensor memory as 8x8 fragments, rounded two
+      // tokens per instruction, transposed by stmatrix into a 1 KiB per-warp block ([token][32
+      // features], the four 16-byte pieces of a row XOR-swizzled against bank conflicts) and leaves
+      // as 16-byte stores.  One 2-byte shared store per element made the tile tail instruction-bound
+      // (about 180 instructions per chunk, now about 70).
       uint16_t* sc0 = tail->transpose[ew];
+      const uint32_t st_addr = smem_u32(sc0) + uint32_t(lane & 7) * 64 + (uint32_t(lane >> 3) ^ ((lane >> 1) & 3u)) * 16;
+      // a chunk as loaded: features 0-15 in v[0..7], 16-31 in v[8..15]
+      auto load_chunk = [&](uint32_t taddr, uint32_t (&v)[16]) {
+        tmem_ld_frag16(taddr, v);
+        tmem_ld_frag16(taddr + (16u << 16), v + 8);
+      };
+      auto store_chunk = [&](const uint32_t (&h)[8]) {  // h[2m + t]: features 8m.., tokens 8t.. of the chunk
+        stmatrix_x4_trans(st_addr, h[0], h[2], h[4], h[6]);
+        stmatrix_x4_trans(st_addr + 8 * 64, h[1], h[3], h[5], h[7]);
+        __syncwarp();
+      };
+      auto piece_of = [&](int piece) -> uint4 {  // token piece/4 of the chunk, features 8*(piece%4) .. +7
+        return *reinterpret_cast<const uint4*>(sc0 + (piece >> 2) * 32 + ((piece & 3) ^ ((piece >> 3) & 3)) * 8);
+      };
       bool released = false;
       auto release = [&]() {
         // every value of this warp's share is in registers: the accumulator may be overwritten
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&tail->acc_empty[buf]));
+        if (lane == 0) mbar_arrive(smem_u32(&tail->acc_empty[buf][0]));
+        released = true;
+      };
+      auto release_half = [&](int half) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&tail->acc_empty[buf][half]));
         released = true;
       };
       if (kMode == kGateUpSwiglu) {
         const int feat_base = fblock * 128 + quarter * 32;
         auto emit = [&](int c, const uint32_t (&g)[16], const uint32_t (&u)[16]) {
           if (c * 16 >= tc.valid) return;  // padding rows only
+          uint32_t h16[8];
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
-            sc0[j * 32 + lane] = to_h16(silu_mul(__uint_as_float(g[j]), __uint_as_float(u[j])), args.fp16);
-          __syncwarp();
+          for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+              const int i = (m >> 1) * 8 + t * 4 + (m & 1) * 2;
+              h16[2 * m + t] = pack_h16x2(silu_mul(__uint_as_float(g[i]), __uint_as_float(u[i])),
+                                          silu_mul(__uint_as_float(g[i + 1]), __uint_as_float(u[i + 1])), args.fp16);
+            }
+          store_chunk(h16);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int piece = lane + 32 * h;  // token piece>>2 of the chunk, features 8*(piece&3) .. +7
@@ -529,7 +605,7 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
             const int feat = feat_base + (piece & 3) * 8;
             if (token < tc.valid && feat < args.out_cols)
               *reinterpret_cast<uint4*>(out + size_t(tc.row0 + token) * args.out_cols + feat) =
-                  *reinterpret_cast<const uint4*>(sc0 + piece * 8);
+                  piece_of(piece);
           }
           __syncwarp();
         };
@@ -538,11 +614,11 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
           uint32_t ga[16], ua[16], gb[16], ub[16];
           const int c2 = c + kChunkStride;
           const bool two = c2 < chunks;
-          tmem_ld16(t0 + c * 16, ga);
-          tmem_ld16(t1 + c * 16, ua);
+          load_chunk(t0 + c * 16, ga);
+          load_chunk(t1 + c * 16, ua);
           if (two) {
-            tmem_ld16(t0 + c2 * 16, gb);
-            tmem_ld16(t1 + c2 * 16, ub);
+            load_chunk(t0 + c2 * 16, gb);
+            load_chunk(t1 + c2 * 16, ub);
           }
           tmem_ld_wait();
           if (c + 2 * kChunkStride >= chunks) release();
@@ -550,49 +626,55 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
           if (two) emit(c2, gb, ub);
         }
       } else {
+        // the two 128-row halves of the tile are drained one after the other, each released as soon as
+        // it is in registers: with one accumulator pair the next tile's products into the first half
+        // run while the second is drained
         const int feat_base = fblock * 256 + quarter * 32;
-        auto emit = [&](int c, const uint32_t (&v0)[16], const uint32_t (&v1)[16]) {
+        auto emit = [&](int c, int half, const uint32_t (&v)[16]) {
           if (c * 16 >= tc.valid) return;
-          // the two 128-row halves of the tile go through the block one after the other
+          uint32_t h16[8];
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const uint32_t (&v)[16] = half == 0 ? v0 : v1;
+          for (int t = 0; t < 2; ++t) {
+            const float2 w = *reinterpret_cast<const float2*>(&tail->tile_weight[par][c * 16 + t * 8 + 2 * (lane & 3)]);
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              sc0[j * 32 + lane] = to_h16(tail->tile_weight[par][c * 16 + j] * __uint_as_float(v[j]), args.fp16);
-            __syncwarp();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int piece = lane + 32 * h;
-              const int a = tail->tile_assign[par][c * 16 + (piece >> 2)];
-              const int feat = feat_base + half * 128 + (piece & 3) * 8;
-              if (a >= 0 && feat < args.out_cols) {
-                // expert parallel: rows of this rank's own tokens go straight into its receive buffer
-                uint16_t* base = (kPush && a < push.own_rows) ? out_own : out;
-                *reinterpret_cast<uint4*>(base + size_t(a) * args.out_cols + feat) =
-                    *reinterpret_cast<const uint4*>(sc0 + piece * 8);
-              }
+            for (int m = 0; m < 4; ++m) {
+              const int i = (m >> 1) * 8 + t * 4 + (m & 1) * 2;
+              h16[2 * m + t] = pack_h16x2(w.x * __uint_as_float(v[i]), w.y * __uint_as_float(v[i + 1]), args.fp16);
             }
-            __syncwarp();
           }
+          store_chunk(h16);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int piece = lane + 32 * h;
+            const int a = tail->tile_assign[par][c * 16 + (piece >> 2)];
+            const int feat = feat_base + half * 128 + (piece & 3) * 8;
+            if (a >= 0 && feat < args.out_cols) {
+              // expert parallel: rows of this rank's own tokens go straight into its receive buffer
+              uint16_t* base = (kPush && a < push.own_rows) ? out_own : out;
+              *reinterpret_cast<uint4*>(base + size_t(a) * args.out_cols + feat) = piece_of(piece);
+            }
+          }
+          __syncwarp();
         };
-        for (int c = cgroup; c < chunks; c += 2 * kChunkStride) {
-          uint32_t a0[16], a1[16], b0[16], b1[16];
-          const int c2 = c + kChunkStride;
-          const bool two = c2 < chunks;
-          tmem_ld16(t0 + c * 16, a0);
-          tmem_ld16(t1 + c * 16, a1);
-          if (two) {
-            tmem_ld16(t0 + c2 * 16, b0);
-            tmem_ld16(t1 + c2 * 16, b1);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t th = half == 0 ? t0 : t1;
+          released = false;
+          for (int c = cgroup; c < chunks; c += 4 * kChunkStride) {
+            uint32_t v[4][16];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (c + u * kChunkStride < chunks) load_chunk(th + (c + u * kChunkStride) * 16, v[u]);
+            tmem_ld_wait();
+            if (c + 4 * kChunkStride >= chunks) release_half(half);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (c + u * kChunkStride < chunks) emit(c + u * kChunkStride, half, v[u]);
           }
-          tmem_ld_wait();
-          if (c + 2 * kChunkStride >= chunks) release();
-          emit(c, a0, a1);
-          if (two) emit(c2, b0, b1);
+          if (!released) release_half(half);
         }
       }
-      if (!released) release();
+      if (kMode == kGateUpSwiglu && !released) release();
       if (kPush) {
         // this warp's share of the token block is stored: count it for the push warps
         __threadfence();

@@ -166,12 +166,14 @@ int check_shape(int64_t tokens, int hidden, int intermediate, int local_experts,
 int run_gemm_stage(int mode, const void* a, int64_t cap, const void* w, int local_experts, int hidden,
                    int intermediate, const int* counts, const int* prefix, const int* sorted,
                    const float* row_scale, void* out, int* status, int device, cudaStream_t stream,
-                   unsigned long long* clock_probe, const FusedDispatch* dispatch, int fp16, const FusedPush* push) {
+                   unsigned long long* clock_probe, const FusedDispatch* dispatch, int fp16, const FusedPush* push,
+                   int early) {
   CUtensorMap map_w;
   TokenMaps maps_t;
   GemmArgs g{};
   g.clock_probe = clock_probe;
   g.fp16 = fp16;
+  g.early = early;
   g.counts = counts;
   g.mtile_prefix = prefix;
   g.sorted_ids = sorted;
@@ -217,11 +219,12 @@ int run_gemm_stage_fp8(int mode, const void* a, const float* a_scale_t, int64_t 
                        const int* counts, const int* prefix, const int* sorted, const float* row_scale,
                        void* out, float* out_scale_t, int* status, int device, cudaStream_t stream,
                        unsigned long long* clock_probe, int pad_rows, const FusedDispatchFp8* dispatch,
-                       const FusedPush* push) {
+                       const FusedPush* push, int early) {
   CUtensorMap map_a, map_b;
   GemmFp8Args g{};
   g.clock_probe = clock_probe;
   g.ue8m0 = g_fp8_ue8m0;
+  g.early = early;
   const bool cols = pad_rows == kPadBf16;  // schedule padded to 16 rows: tokens-on-columns kernel
   TokenMaps maps_t;
   if (cols) {
@@ -413,6 +416,7 @@ static int moe_forward_16bit(int fp16, const void* hidden_states, const void* w1
   // the row gather runs inside the gate/up GEMM kernel (dispatch warps); the sort resets its counters
   sched.clear = reinterpret_cast<int*>(ws + l.granules);
   sched.clear_ints = l.granule_bytes / 4;
+  sched.chained = chain_forward(tokens * topk, local_experts, hidden, intermediate, 2);
   mark_stage(0, s);
   if ((rc = launch_align(topk_ids, tokens * topk, expert_map, local_experts, sched, cap,
                          reinterpret_cast<int*>(ws + l.scratch), s))) return rc;
@@ -431,13 +435,16 @@ static int moe_forward_16bit(int fp16, const void* hidden_states, const void* w1
   mark_stage(2, s);
   if ((rc = run_gemm_stage(kGateUpSwiglu, xg, cap, w1, local_experts, hidden, intermediate, sched.counts,
                            sched.mtile_prefix, sched.sorted_ids, nullptr, act, status, device, s,
-                             reinterpret_cast<unsigned long long*>(status + 8), &disp, fp16))) return rc;
+                             reinterpret_cast<unsigned long long*>(status + 8), &disp, fp16, nullptr,
+                           sched.chained ? kEarlyBeforeTokens : kEarlyOff))) return rc;
   mark_stage(3, s);
   if ((rc = run_gemm_stage(kDownWeighted, act, cap, w2, local_experts, hidden, intermediate, sched.counts,
                            sched.mtile_prefix, sched.sorted_ids, topk_weights, y, status, device, s,
-                             reinterpret_cast<unsigned long long*>(status + 12), nullptr, fp16))) return rc;
+                             reinterpret_cast<unsigned long long*>(status + 12), nullptr, fp16, nullptr,
+                           sched.chained ? kEarlyBeforePrevious : kEarlyOff))) return rc;
   mark_stage(4, s);
-  rc = launch_combine_bf16(y, sched.inverse, int(tokens), topk, hidden, reinterpret_cast<__nv_bfloat16*>(out), s, fp16);
+  rc = launch_combine_bf16(y, sched.inverse, int(tokens), topk, hidden, reinterpret_cast<__nv_bfloat16*>(out), s, fp16,
+                           sched.chained);
   mark_stage(5, s);
   return rc;
 }
@@ -534,6 +541,7 @@ int mb200_moe_forward_fp8(const void* hidden_states, const void* w1, const void*
     sched.clear = reinterpret_cast<int*>(ws + l.granules);
     sched.clear_ints = l.granule_bytes / 4;
   }
+  sched.chained = chain_forward(tokens * topk, local_experts, hidden, intermediate, 1);
   mark_stage(0, s);
   if ((rc = launch_align(topk_ids, tokens * topk, expert_map, local_experts, sched, cap,
                          reinterpret_cast<int*>(ws + l.scratch), s))) return rc;
@@ -543,7 +551,7 @@ int mb200_moe_forward_fp8(const void* hidden_states, const void* w1, const void*
   uint8_t* xq_tok = reinterpret_cast<uint8_t*>(ws + l.xq_tok);
   float* xs_tok = reinterpret_cast<float*>(ws + l.xs_tok);
   if ((rc = launch_group_quant_fp8(reinterpret_cast<const __nv_bfloat16*>(hidden_states), tokens, hidden, xq_tok,
-                                   xs_tok, hidden / 128, 0, s, g_fp8_ue8m0))) return rc;
+                                   xs_tok, hidden / 128, 0, s, g_fp8_ue8m0, sched.chained))) return rc;
   PeerTable self_q{}, self_s{};
   self_q.ptr[0] = xq_tok;
   self_s.ptr[0] = xs_tok;
@@ -569,13 +577,16 @@ int mb200_moe_forward_fp8(const void* hidden_states, const void* w1, const void*
   if ((rc = run_gemm_stage_fp8(kGateUpSwiglu, xq, xs_t, cap, w1, w1_scale, local_experts, hidden, intermediate,
                                sched.counts, sched.mtile_prefix, sched.sorted_ids, nullptr, actq, acts_t, status,
                                device, s, reinterpret_cast<unsigned long long*>(status + 8), pad,
-                               disp.enabled ? &disp : nullptr))) return rc;
+                               disp.enabled ? &disp : nullptr, nullptr,
+                               !sched.chained ? kEarlyOff : disp.enabled ? kEarlyBeforeTokens : kEarlyBeforePrevious))) return rc;
   mark_stage(3, s);
   if ((rc = run_gemm_stage_fp8(kDownWeighted, actq, acts_t, cap, w2, w2_scale, local_experts, hidden, intermediate,
                                sched.counts, sched.mtile_prefix, sched.sorted_ids, topk_weights, y, nullptr, status,
-                               device, s, reinterpret_cast<unsigned long long*>(status + 12), pad))) return rc;
+                               device, s, reinterpret_cast<unsigned long long*>(status + 12), pad, nullptr, nullptr,
+                               sched.chained ? kEarlyBeforePrevious : kEarlyOff))) return rc;
   mark_stage(4, s);
-  rc = launch_combine_bf16(y, sched.inverse, int(tokens), topk, hidden, reinterpret_cast<__nv_bfloat16*>(out), s);
+  rc = launch_combine_bf16(y, sched.inverse, int(tokens), topk, hidden, reinterpret_cast<__nv_bfloat16*>(out), s, 0,
+                           sched.chained);
   mark_stage(5, s);
   return rc;
 }

@@ -223,6 +223,14 @@ __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, Wa
   }
 }
 
+// ---- programmatic dependent launch -----------------------------------------------
+// A kernel launched with launch_chained() may start while the kernel before it on the stream is
+// still running (once all of that kernel's blocks have called pdl_trigger() or exited).
+// pdl_wait() returns when the kernels before it have completed and their writes are visible;
+// every such kernel calls it before it exits, so completion stays transitive along the stream.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- TMA ------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");

@@ -204,7 +204,11 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
     tmem_alloc(smem_u32(&tail->tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  for (int i = threadIdx.x; i <= E; i += kThreads) tail->prefix[i] = args.mtile_prefix[i];
+  // Up to here nothing was read that the kernels ahead on the stream write.  The schedule may be
+  // older than the kernel directly ahead (down GEMM: it is complete before the gate/up GEMM starts),
+  // then this CTA goes on to its first weights while that kernel's last tiles finish elsewhere.
+  if (args.early != kEarlyBeforePrevious) pdl_wait();
+  for (int i = threadIdx.x; i <= E; i += kThreads) tail->prefix[i] = __ldcg(args.mtile_prefix + i);
   __syncthreads();
   // largest expert segment -> token box, stage geometry
   {
@@ -254,10 +258,13 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
   const int total_tiles = tail->tb_prefix[E] * n_fgroups;
   const uint32_t acc1_off = geo.acc_bufs == 2 ? 128u : 256u;  // column of the second accumulator
   WaitCtx ctx{&tail->abort_flag, args.status, wait_limit_ns(args.status)};
+  if (args.early == kEarlyBeforePrevious && warp != 0) pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane < kTokenBoxes) prefetch_tmap(&maps_t.m[lane]);
+    if (args.early == kEarlyBeforePrevious && worker >= total_tiles) pdl_wait();  // no first tile to wait in
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -265,6 +272,28 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
       const TileCoord tc = decode_tile(tile, tail, args.counts, E, n_fgroups, geo.tb_rows);
       const int fblock = tc.fblock;
       const int w_row = tc.expert * args.b_rows_per_expert;
+      auto load_weights = [&](int kb, int to_stage) {
+        const uint32_t bar = smem_u32(&tail->full[to_stage]);
+        const uint32_t w_dst = ring_addr + to_stage * geo.stage_bytes;
+        const int kcol = kb * 64;
+        mbar_expect_tx(bar, uint32_t(kWeightBytes + tc.ntok * 128));
+        if (kMode == kGateUpSwiglu) {
+          tma_load_2d(w_dst, &map_w, kcol, w_row + fblock * 128, bar);
+          tma_load_2d(w_dst + kWeightBytes / 2, &map_w, kcol, w_row + args.b_half_offset + fblock * 128, bar);
+        } else {
+          tma_load_2d(w_dst, &map_w, kcol, w_row + fblock * 256, bar);
+        }
+      };
+      int ahead = 0;  // K steps whose weights are already on their way
+      if (args.early != kEarlyOff && tile == worker) {
+        // first tile: the stages are empty and the weights depend on nothing but the schedule,
+        // so they are requested before the wait for the tokens
+        ahead = geo.stages < args.k_iters ? geo.stages : args.k_iters;
+        if (lane == 0)
+          for (int kb = 0; kb < ahead; ++kb) load_weights(kb, kb);
+        __syncwarp();
+        if (args.early == kEarlyBeforePrevious) pdl_wait();
+      }
       if (kMode == kGateUpSwiglu && disp.enabled) {
         // all 16-row granules of this token block must have been dispatched
         const int g0 = tc.row0 / kPad, ng = tc.ntok / kPad;  // ng <= 16
@@ -295,18 +324,10 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
         ok = mbar_wait(smem_u32(&tail->empty[stage]), phase ^ 1, ctx, 1);
         if (!ok) break;
         if (lane == 0) {
+          if (kb >= ahead) load_weights(kb, stage);
           const uint32_t bar = smem_u32(&tail->full[stage]);
-          const uint32_t w_dst = ring_addr + stage * geo.stage_bytes;
-          const uint32_t t_dst = w_dst + kWeightBytes;
+          const uint32_t t_dst = ring_addr + stage * geo.stage_bytes + kWeightBytes;
           const int kcol = kb * 64;
-          mbar_expect_tx(bar, uint32_t(kWeightBytes + tc.ntok * 128));
-          if (kMode == kGateUpSwiglu) {
-            tma_load_2d(w_dst, &map_w, kcol, w_row + fblock * 128, bar);
-            tma_load_2d(w_dst + kWeightBytes / 2, &map_w, kcol,
-                        w_row + args.b_half_offset + fblock * 128, bar);
-          } else {
-            tma_load_2d(w_dst, &map_w, kcol, w_row + fblock * 256, bar);
-          }
           // exactly ntok token rows: one box per set bit of ntok/16 (largest first), so a
           // 144-token tile moves 18 KB of tokens, not the 32 KB of the launch's largest box
           const int nb16 = tc.ntok >> 4;
@@ -730,20 +751,12 @@ int launch_grouped_gemm_bf16(GemmMode mode, const CUtensorMap& map_w, const Toke
   }
   const int sms = device_sm_count(device);
   MB200_REQUIRE(sms > 0, kCudaError, "grouped_gemm: cannot read the SM count of device %d", device);
-  if (dispatch.enabled == kDispatchFused || push.enabled) {
-    // the tile loader waits for rows that other CTAs' dispatch warps deliver, the push warps
-    // for tiles that other CTAs compute: all CTAs must be resident, which a cooperative
-    // launch guarantees (or refuses)
-    void* params[] = {const_cast<CUtensorMap*>(&map_w), const_cast<TokenMaps*>(&maps_t),
-                      const_cast<GemmArgs*>(&args), const_cast<FusedDispatch*>(&dispatch),
-                      const_cast<FusedPush*>(&push)};
-    MB200_CHECK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(sms), dim3(kThreads),
-                                                 params, kSmemBytes, stream));
-  } else {
-    kernel<<<sms, kThreads, kSmemBytes, stream>>>(map_w, maps_t, args, dispatch, push);
-    MB200_CHECK_CUDA(cudaGetLastError());
-  }
-  return kOk;
+  // the tile loader waits for rows that other CTAs' dispatch warps deliver, the push warps
+  // for tiles that other CTAs compute: all CTAs must be resident, which a cooperative
+  // launch guarantees (or refuses)
+  const bool cooperative = dispatch.enabled == kDispatchFused || push.enabled;
+  return launch_chained(kernel, dim3(sms), kThreads, kSmemBytes, stream, cooperative,
+                        !cooperative && args.early != kEarlyOff, map_w, maps_t, args, dispatch, push);
 }
 
 }  // namespace mb200

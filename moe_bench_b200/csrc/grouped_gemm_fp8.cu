@@ -167,7 +167,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
     tmem_alloc(smem_u32(&tail->tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  for (int i = threadIdx.x; i <= args.num_experts; i += kThreads) tail->prefix[i] = args.mtile_prefix[i];
+  // Up to here nothing was read that the kernels ahead on the stream write.  The schedule may be
+  // older than the kernel directly ahead (down GEMM: it is complete before the gate/up GEMM starts),
+  // then this CTA goes on to its first weights while that kernel's last tiles finish elsewhere.
+  if (args.early != kEarlyBeforePrevious) pdl_wait();
+  for (int i = threadIdx.x; i <= args.num_experts; i += kThreads) tail->prefix[i] = __ldcg(args.mtile_prefix + i);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -177,6 +181,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
   const int total_tiles = tail->prefix[args.num_experts] * args.n_tiles;
   const int k_blocks = args.k_blocks;
   WaitCtx ctx{&tail->abort_flag, args.status, wait_limit_ns(args.status)};
+  if (args.early == kEarlyBeforePrevious && warp != 0) pdl_wait();
+  pdl_trigger();
 
   // Each role's code sits inside the branch that re-sizes its warpgroup's registers, so the
   // compiler knows which budget applies where.
@@ -184,6 +190,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegSplit<kMode>::kHelper));
   if (warp == 0) {
     // ---------------- TMA producer ----------------
+    if (args.early == kEarlyBeforePrevious && int(blockIdx.x) >= total_tiles) pdl_wait();  // no first tile to wait in
     int stage = 0;
     uint32_t phase = 0;
     uint32_t slot = 0;  // scale slot of the K block being loaded
@@ -191,6 +198,28 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
     for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
       TileCoord tc = decode_tile(tile, tail->prefix, args.counts, args.num_experts, args.n_tiles);
       const int b_row = tc.expert * args.b_rows_per_expert;
+      auto load_weights = [&](int kb, int to_stage) {
+        const uint32_t bar = smem_u32(&tail->full[to_stage]);
+        const uint32_t b_dst = tiles_addr + to_stage * kStageBytes + kABytes;
+        const int kcol = kb * 128;
+        mbar_expect_tx(bar, kStageBytes + kTileM * 4);
+        if (kMode == kGateUpSwiglu) {
+          tma_load_2d(b_dst, &map_b, kcol, b_row + tc.n_tile * 128, bar);
+          tma_load_2d(b_dst + kBBytes / 2, &map_b, kcol, b_row + args.b_half_offset + tc.n_tile * 128, bar);
+        } else {
+          tma_load_2d(b_dst, &map_b, kcol, b_row + tc.n_tile * 256, bar);
+        }
+      };
+      int ahead = 0;  // K blocks whose weights are already on their way
+      if (args.early != kEarlyOff && tile == int(blockIdx.x)) {
+        // first tile: the stages are empty and the weights depend on nothing but the schedule,
+        // so they are requested before the wait for the tokens
+        ahead = kStages < k_blocks ? kStages : k_blocks;
+        if (lane == 0)
+          for (int kb = 0; kb < ahead; ++kb) load_weights(kb, kb);
+        __syncwarp();
+        if (args.early == kEarlyBeforePrevious) pdl_wait();
+      }
       if (kMode == kGateUpSwiglu && disp.enabled) {
         // the eight 16-row granules of this token tile must have been dispatched
         const int g0 = tc.row0 / 16;
@@ -221,20 +250,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
         if (!ok) break;
         if (lane == 0) {
           const uint32_t bar = smem_u32(&tail->full[stage]);
-          const uint32_t a_dst = tiles_addr + stage * kStageBytes;
-          const uint32_t b_dst = a_dst + kABytes;
-          const int kcol = kb * 128;
-          mbar_expect_tx(bar, kStageBytes + kTileM * 4);
+          if (kb >= ahead) load_weights(kb, stage);
           tma_load_1d(smem_u32(tail->ascale[slot]), args.a_scale_t + size_t(kb) * args.row_capacity + tc.row0,
                       kTileM * 4, bar);
-          tma_load_2d(a_dst, &map_a, kcol, tc.row0, bar);
-          if (kMode == kGateUpSwiglu) {
-            tma_load_2d(b_dst, &map_b, kcol, b_row + tc.n_tile * 128, bar);
-            tma_load_2d(b_dst + kBBytes / 2, &map_b, kcol,
-                        b_row + args.b_half_offset + tc.n_tile * 128, bar);
-          } else {
-            tma_load_2d(b_dst, &map_b, kcol, b_row + tc.n_tile * 256, bar);
-          }
+          tma_load_2d(tiles_addr + stage * kStageBytes, &map_a, kb * 128, tc.row0, bar);
         }
         __syncwarp();
         if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -596,19 +615,11 @@ int launch_grouped_gemm_fp8(GemmMode mode, const CUtensorMap& map_a, const CUten
                                           int(kSmemBytes)));
     if (device >= 0 && device < kMaxDevices) configured[device][mode].store(true, std::memory_order_release);
   }
-  if (dispatch.enabled || push.enabled) {
-    // the tile loader waits for rows that other CTAs' dispatch warps deliver, the push warps for
-    // tiles that other CTAs compute: all CTAs must be resident (a cooperative launch guarantees it)
-    void* params[] = {const_cast<CUtensorMap*>(&map_a), const_cast<CUtensorMap*>(&map_b),
-                      const_cast<GemmFp8Args*>(&args), const_cast<FusedDispatchFp8*>(&dispatch),
-                      const_cast<FusedPush*>(&push)};
-    MB200_CHECK_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), dim3(sms), dim3(kThreads),
-                                                 params, kSmemBytes, stream));
-  } else {
-    kernel<<<sms, kThreads, kSmemBytes, stream>>>(map_a, map_b, args, dispatch, push);
-    MB200_CHECK_CUDA(cudaGetLastError());
-  }
-  return kOk;
+  // the tile loader waits for rows that other CTAs' dispatch warps deliver, the push warps for
+  // tiles that other CTAs compute: all CTAs must be resident (a cooperative launch guarantees it)
+  const bool cooperative = dispatch.enabled || push.enabled;
+  return launch_chained(kernel, dim3(sms), kThreads, kSmemBytes, stream, cooperative,
+                        !cooperative && args.early != kEarlyOff, map_a, map_b, args, dispatch, push);
 }
 
 }  // namespace mb200

@@ -174,7 +174,11 @@ grouped_gemm_fp8_cols_kernel(const __grid_constant__ CUtensorMap map_w,
     tmem_alloc(smem_u32(&tail->tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  for (int i = threadIdx.x; i <= E; i += kThreads) tail->prefix[i] = args.mtile_prefix[i];
+  // Up to here nothing was read that the kernels ahead on the stream write.  The schedule is
+  // complete before the kernel directly ahead starts its blocks (row gather, gate/up GEMM), so in a
+  // forward this CTA goes on to its first weights while that kernel finishes elsewhere.
+  if (args.early != kEarlyBeforePrevious) pdl_wait();
+  for (int i = threadIdx.x; i <= E; i += kThreads) tail->prefix[i] = __ldcg(args.mtile_prefix + i);
   __syncthreads();
   {
     int mx = 0;
@@ -220,11 +224,14 @@ grouped_gemm_fp8_cols_kernel(const __grid_constant__ CUtensorMap map_w,
   const uint32_t tmem_base = tail->tmem_base;
   const int total_tiles = tail->tb_prefix[E] * args.n_tiles;
   WaitCtx ctx{&tail->abort_flag, args.status, wait_limit_ns(args.status)};
+  if (args.early == kEarlyBeforePrevious && warp != 0) pdl_wait();
+  pdl_trigger();
 
   if (warp == 0) {
     // ---------------- TMA producer: one stage = one 128-deep K block ----------------
     const CUtensorMap* map_t = &maps_t.m[geo.box_index];
     if (lane == 0) prefetch_tmap(map_t);
+    if (args.early == kEarlyBeforePrevious && int(blockIdx.x) >= total_tiles) pdl_wait();  // no first tile to wait in
     int stage = 0;
     uint32_t phase = 0;
     int slot = 0;  // scale slot of the K block being loaded
@@ -232,25 +239,38 @@ grouped_gemm_fp8_cols_kernel(const __grid_constant__ CUtensorMap map_w,
     for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
       const TileCoord tc = decode_tile(tile, tail, args.counts, E, args.n_tiles);
       const int w_row = tc.expert * args.b_rows_per_expert;
+      auto load_weights = [&](int kb, int to_stage) {
+        const uint32_t bar = smem_u32(&tail->full[to_stage]);
+        const uint32_t w_dst = ring_addr + to_stage * geo.stage_bytes;
+        const int kcol = kb * 128;
+        mbar_expect_tx(bar, uint32_t(geo.stage_bytes + tc.ntok * 4));
+        if (kMode == kGateUpSwiglu) {
+          tma_load_2d(w_dst, &map_w, kcol, w_row + tc.fblock * 128, bar);
+          tma_load_2d(w_dst + kWeightBytes / 2, &map_w, kcol, w_row + args.b_half_offset + tc.fblock * 128, bar);
+        } else {
+          tma_load_2d(w_dst, &map_w, kcol, w_row + tc.fblock * 256, bar);
+        }
+      };
+      int ahead = 0;  // K blocks whose weights are already on their way
+      if (args.early != kEarlyOff && tile == int(blockIdx.x)) {
+        // first tile: the stages are empty and the weights depend on nothing but the schedule,
+        // so they are requested before the wait for the tokens
+        ahead = geo.stages < k_blocks ? geo.stages : k_blocks;
+        if (lane == 0)
+          for (int kb = 0; kb < ahead; ++kb) load_weights(kb, kb);
+        __syncwarp();
+        if (args.early == kEarlyBeforePrevious) pdl_wait();
+      }
       for (int kb = 0; kb < k_blocks; ++kb) {
         ok = mbar_wait(smem_u32(&tail->empty[stage]), phase ^ 1, ctx, 1);
         if (!ok) break;
         if (lane == 0) {
           const uint32_t bar = smem_u32(&tail->full[stage]);
-          const uint32_t w_dst = ring_addr + stage * geo.stage_bytes;
-          const uint32_t t_dst = w_dst + kWeightBytes;
-          const int kcol = kb * 128;
-          mbar_expect_tx(bar, uint32_t(geo.stage_bytes + tc.ntok * 4));
+          const uint32_t t_dst = ring_addr + stage * geo.stage_bytes + kWeightBytes;
+          if (kb >= ahead) load_weights(kb, stage);
           tma_load_1d(smem_u32(tail->ascale + slot * geo.tb_rows),
                       args.a_scale_t + size_t(kb) * args.row_capacity + tc.row0, uint32_t(tc.ntok * 4), bar);
-          if (kMode == kGateUpSwiglu) {
-            tma_load_2d(w_dst, &map_w, kcol, w_row + tc.fblock * 128, bar);
-            tma_load_2d(w_dst + kWeightBytes / 2, &map_w, kcol,
-                        w_row + args.b_half_offset + tc.fblock * 128, bar);
-          } else {
-            tma_load_2d(w_dst, &map_w, kcol, w_row + tc.fblock * 256, bar);
-          }
-          tma_load_2d(t_dst, map_t, kcol, tc.row0, bar);
+          tma_load_2d(t_dst, map_t, kb * 128, tc.row0, bar);
         }
         __syncwarp();
         if (++stage == geo.stages) { stage = 0; phase ^= 1; }
@@ -483,9 +503,7 @@ int launch_grouped_gemm_fp8_cols(GemmMode mode, const CUtensorMap& map_w, const 
                                           int(kSmemBytes)));
     if (device >= 0 && device < kMaxDevices) configured[device][mode].store(true, std::memory_order_release);
   }
-  kernel<<<sms, kThreads, kSmemBytes, stream>>>(map_w, maps_t, args);
-  MB200_CHECK_CUDA(cudaGetLastError());
-  return kOk;
+  return launch_chained(kernel, dim3(sms), kThreads, kSmemBytes, stream, false, args.early != kEarlyOff, map_w, maps_t, args);
 }
 
 }  // namespace mb200

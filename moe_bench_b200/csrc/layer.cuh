@@ -15,6 +15,45 @@ constexpr int kMaxDevices = 64;    // device ordinals the per-device caches cove
 // SM count of a device, cached (thread-safe); 0 if it cannot be read.
 int device_sm_count(int device);
 
+// Launch of a kernel that calls pdl_wait(): cooperative where its blocks wait for one another, and,
+// `chained`, with the programmatic-serialization attribute.
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, bool cooperative,
+                   bool chained, A&&... args) {
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (chained) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cooperative) {
+    attr[n].id = cudaLaunchAttributeCooperative;
+    attr[n++].val.cooperative = 1;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  MB200_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  return kOk;
+}
+
+// Whether a forward's kernels are chained.  Overlapping prologues, launch gaps and the first weight
+// loads saves about 10 us; it is done where the weights stream for up to 0.3 ms and the batch is small.
+// One B200, chained against not: 0.35 GB of weights 105 / 117 us, 0.7 GB 140 / 148 us, 1.4 GB 271 /
+// 283 us (512 tokens: 310 / 315 us); past that there is nothing to gain (2.5 GB 465 / 465 us, 2.8 GB
+// 445 / 443 us), and large batches lose (32768 assignments 885 / 869 us, 11 GB 1911 / 1878 us).
+constexpr int64_t kChainMaxWeightBytes = int64_t(2) << 30;
+constexpr int64_t kChainMaxAssignments = 8192;
+inline bool chain_forward(int64_t assignments, int experts, int hidden, int intermediate, int elem_bytes) {
+  const int64_t touched = assignments < experts ? assignments : experts;
+  return assignments <= kChainMaxAssignments &&
+         touched * 3 * hidden * intermediate * elem_bytes <= kChainMaxWeightBytes;
+}
+
 constexpr int kMaxPeers = 16;
 struct PeerTable {
   void* ptr[kMaxPeers];  // one pointer per rank, valid in this process
@@ -29,6 +68,7 @@ struct Schedule {
   int pad_rows;       //        granule every expert segment is padded to
   int* clear = nullptr;    // counters the sort sets to zero on its way (the GEMMs' arrival counters)
   int64_t clear_ints = 0;
+  bool chained = false;    // the kernels of this forward overlap (launch_chained)
 };
 
 // ---- route_align.cu ---------------------------------------------------------------
@@ -43,7 +83,8 @@ int launch_align(const int* topk_ids, int64_t assignments, const int* expert_map
 // ---- rows.cu ------------------------------------------------------------------------
 // y and out are 16-bit (bf16, or fp16 when fp16 != 0); fp32 sum.
 int launch_combine_bf16(const __nv_bfloat16* y, const int* inverse, int tokens, int topk,
-                        int hidden, __nv_bfloat16* out, cudaStream_t stream, int fp16 = 0);
+                        int hidden, __nv_bfloat16* out, cudaStream_t stream, int fp16 = 0,
+                        bool chained = false);
 // Tensor parallel combine: sum over k and store the row into the owner's `partial` plane of this
 // rank; then the owner's sum over its W local planes.
 int launch_combine_push(const __nv_bfloat16* y, int all_tokens, int tokens_per_rank, int topk, int hidden,
@@ -51,13 +92,21 @@ int launch_combine_push(const __nv_bfloat16* y, int all_tokens, int tokens_per_r
 int launch_sum_planes(const __nv_bfloat16* partial, int tokens, int world, int hidden, __nv_bfloat16* out,
                       cudaStream_t stream, int fp16 = 0);
 // Per-row, per-128-group e4m3 quantisation.  scales_t is [K/128][scale_ld] (group-major).
+// chained: the kernel ahead on the stream neither writes x nor uses q and scales, and was itself
+// launched after x was complete: the two may overlap.
 int launch_group_quant_fp8(const __nv_bfloat16* x, int64_t rows, int hidden, uint8_t* q,
-                           float* scales, int64_t scale_ld, int transposed, cudaStream_t stream, int ue8m0 = 0);
+                           float* scales, int64_t scale_ld, int transposed, cudaStream_t stream, int ue8m0 = 0,
+                           bool chained = false);
 // Activation scale format the calling thread selected (mb200_set_fp8_scale_format): 0 = fp32
 // amax/448, 1 = rounded up to a power of two.
 int fp8_scale_ue8m0();
 
 // ---- grouped_gemm.cu -----------------------------------------------------------------
+// When a CTA requests the weights of its first K steps: with the tokens; before it waits for the
+// tokens; or (schedule complete before the kernel ahead started its blocks) before that kernel has
+// completed.  The last two are launched chained, except a cooperative kernel: its blocks wait for one
+// another and must be placed together, whatever else starts early on other streams.
+enum EarlyWeights : int { kEarlyOff = 0, kEarlyBeforeTokens = 1, kEarlyBeforePrevious = 2 };
 struct GemmArgs {
   const int* counts;
   const int* mtile_prefix;  // cumulative 16-row blocks
@@ -73,6 +122,7 @@ struct GemmArgs {
   int* status;
   unsigned long long* clock_probe;  // optional [2]: SM cycles and nanoseconds CTA 0 spent in the kernel
   int fp16;                // operands and outputs are fp16 instead of bf16
+  int early;               // EarlyWeights
 };
 enum GemmMode : int { kGateUpSwiglu = 0, kDownWeighted = 1 };
 // Dispatch fused into the gate/up GEMM: extra warps of every CTA fill the sorted
@@ -146,6 +196,7 @@ struct GemmFp8Args {
   int* status;
   unsigned long long* clock_probe;  // optional [2]: SM cycles and nanoseconds CTA 0 spent in the kernel
   int ue8m0;                  // gate/up: re-quantise the activations with power-of-two scales
+  int early;                  // EarlyWeights
 };
 // Dispatch fused into the fp8 gate/up GEMM (128-row-tile kernel): two helper warps of every CTA
 // fill the sorted row buffer with the tokens' e4m3 rows and their 1x128 scales, 16-row granule by
@@ -211,13 +262,14 @@ int run_gemm_stage(int mode, const void* a, int64_t cap, const void* w, int loca
                    int intermediate, const int* counts, const int* prefix, const int* sorted,
                    const float* row_scale, void* out, int* status, int device, cudaStream_t stream,
                    unsigned long long* clock_probe = nullptr, const FusedDispatch* dispatch = nullptr,
-                   int fp16 = 0, const FusedPush* push = nullptr);
+                   int fp16 = 0, const FusedPush* push = nullptr, int early = 0);
 int run_gemm_stage_fp8(int mode, const void* a, const float* a_scale_t, int64_t cap, const void* w,
                        const float* w_scale, int local_experts, int hidden, int intermediate,
                        const int* counts, const int* prefix, const int* sorted, const float* row_scale,
                        void* out, float* out_scale_t, int* status, int device, cudaStream_t stream,
                        unsigned long long* clock_probe = nullptr, int pad_rows = kTileM,
-                       const FusedDispatchFp8* dispatch = nullptr, const FusedPush* push = nullptr);
+                       const FusedDispatchFp8* dispatch = nullptr, const FusedPush* push = nullptr,
+                       int early = 0);
 void mark_stage(int i, cudaStream_t s);
 
 // ---- tensormap.cu ----------------------------------------------------------------------

@@ -102,6 +102,8 @@ __global__ void gather_rows_peer_fp8_kernel(PeerTable xq, PeerTable xs, int rank
                                             const int* __restrict__ mtile_prefix, int local_experts,
                                             int groups_per_row, uint4* __restrict__ out_q,
                                             float* __restrict__ out_scales_t, int64_t row_capacity, int pad) {
+  pdl_wait();
+  pdl_trigger();  // after the wait: the kernel that follows may rely on the schedule
   int64_t rows = int64_t(__ldg(mtile_prefix + local_experts)) * pad;
   if (rows > row_capacity) rows = row_capacity;
   const int warps_per_block = blockDim.x >> 5;
@@ -221,11 +223,9 @@ int launch_gather_rows_peer_fp8(const PeerTable& x, const PeerTable& xs, int ran
   const int threads = 256;
   const int blocks = grid_for_rows(row_capacity * 32, threads, 16);
   MB200_REQUIRE(hidden % 128 == 0, kUnsupportedShape, "dispatch: hidden=%d must be a multiple of 128", hidden);
-  gather_rows_peer_fp8_kernel<<<blocks, threads, 0, stream>>>(
-      x, xs, rank, world, tokens, topk, sched.sorted_ids, sched.mtile_prefix, local_experts, hidden / 128,
-      reinterpret_cast<uint4*>(out_rows), out_scales_t, row_capacity, sched.pad_rows);
-  MB200_CHECK_CUDA(cudaGetLastError());
-  return kOk;
+  return launch_chained(gather_rows_peer_fp8_kernel, dim3(blocks), threads, 0, stream, false, sched.chained, x, xs, rank, world,
+                        tokens, topk, sched.sorted_ids, sched.mtile_prefix, local_experts, hidden / 128,
+                        reinterpret_cast<uint4*>(out_rows), out_scales_t, row_capacity, sched.pad_rows);
 }
 
 int launch_reduce_partials(const PeerTable& partial, int rank, int world, int tokens, int topk,

@@ -178,6 +178,7 @@ __global__ void align_count_kernel(const int* __restrict__ topk_ids, const int* 
                                    int64_t assignments, int local_experts, int64_t chunk,
                                    int* __restrict__ block_hist) {
   extern __shared__ int hist[];  // [E]
+  pdl_trigger();
   for (int e = threadIdx.x; e < local_experts; e += blockDim.x) hist[e] = 0;
   __syncthreads();
   const int64_t unit = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -207,6 +208,7 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
   int* prefix = base + E;
   int* part = prefix + E + 1;
   const int nb = gridDim.x;
+  pdl_trigger();
 
   // counters of the kernels that follow (arrivals per granule / token block)
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < clear_ints; i += int64_t(nb) * blockDim.x)
@@ -222,6 +224,7 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
   walk_chunk(topk_ids, expert_map, begin, end, E, [&](int64_t, int slot, int before, unsigned peers) {
     if (slot >= 0 && before == 0) running[slot] += __popc(peers);
   });
+  pdl_wait();  // the blocks' histograms
   __syncthreads();
 
   // 2. total[e] over all blocks, base[e] over the blocks before this one.  Thread groups of E
@@ -376,7 +379,13 @@ int launch_align(const int* topk_ids, int64_t assignments, const int* expert_map
     MB200_CHECK_CUDA(cudaGetLastError());
   }
   const size_t smem = size_t(sh.warps * local_experts + 3 * local_experts + 1 + 2 * threads) * sizeof(int);
-  align_scatter_kernel<<<sh.blocks, threads, smem, stream>>>(
+  // The first kernel of the sort is an ordinary launch: what came before it on the stream is
+  // complete, so the second may overlap the first up to the histograms.
+  if (sh.blocks > 1)
+    return launch_chained(align_scatter_kernel, dim3(sh.blocks), threads, smem, stream, false, sched.chained, topk_ids, expert_map,
+                          assignments, local_experts, sh.chunk, scratch, sched.counts, sched.mtile_prefix,
+                          sched.sorted_ids, sched.inverse, row_capacity, pad, sched.clear, sched.clear_ints);
+  align_scatter_kernel<<<1, threads, smem, stream>>>(
       topk_ids, expert_map, assignments, local_experts, sh.chunk, scratch, sched.counts, sched.mtile_prefix,
       sched.sorted_ids, sched.inverse, row_capacity, pad, sched.clear, sched.clear_ints);
   MB200_CHECK_CUDA(cudaGetLastError());

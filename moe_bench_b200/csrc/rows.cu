@@ -29,6 +29,7 @@ template <int kVecs, int kRows>
 __global__ void __launch_bounds__(256)
 combine_bf16_kernel(const uint4* __restrict__ y, const int* __restrict__ inverse, int tokens, int topk,
                     int vec_per_row, int runs, uint4* __restrict__ out, int fp16) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t total = int64_t(tokens) * runs;
   for (int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; i < total;
@@ -158,7 +159,9 @@ __device__ __forceinline__ float quantize_slice16(const uint4& a, const uint4& b
 template <bool kUe8m0>
 __global__ void group_quant_fp8_kernel(const uint4* __restrict__ x, int64_t rows, int groups_per_row,
                                        uint2* __restrict__ q, float* __restrict__ scales,
-                                       int64_t scale_ld, int transposed) {
+                                       int64_t scale_ld, int transposed, int beside_previous) {
+  pdl_trigger();
+  if (!beside_previous) pdl_wait();
   const bool wide = (reinterpret_cast<uintptr_t>(q) & 15) == 0;  // a caller's buffer may be 8-byte aligned
   const int64_t total_groups = rows * groups_per_row;
   const int sub = threadIdx.x & 7;
@@ -181,6 +184,8 @@ __global__ void group_quant_fp8_kernel(const uint4* __restrict__ x, int64_t rows
       else scales[row * scale_ld + grp] = scale;
     }
   }
+  // whoever waits for this kernel also waits for the one before it
+  if (beside_previous) pdl_wait();
 }
 
 int grid_for(int64_t work_items, int threads, int device_sms, int waves) {
@@ -199,7 +204,7 @@ int sm_count() {
 }  // namespace
 
 int launch_combine_bf16(const __nv_bfloat16* y, const int* inverse, int tokens, int topk, int hidden,
-                        __nv_bfloat16* out, cudaStream_t stream, int fp16) {
+                        __nv_bfloat16* out, cudaStream_t stream, int fp16, bool chained) {
   MB200_REQUIRE(hidden % 8 == 0, kUnsupportedShape, "combine: hidden=%d must be a multiple of 8", hidden);
   if (tokens == 0) return kOk;
   const int threads = 256, sms = sm_count();
@@ -208,10 +213,8 @@ int launch_combine_bf16(const __nv_bfloat16* y, const int* inverse, int tokens, 
   const int runs = wide ? (vecs + 127) / 128 : (vecs + 31) / 32;
   const int blocks = grid_for(int64_t(tokens) * runs * 32, threads, sms, 16);
   auto kernel = wide ? combine_bf16_kernel<4, 4> : combine_bf16_kernel<1, 8>;
-  kernel<<<blocks, threads, 0, stream>>>(reinterpret_cast<const uint4*>(y), inverse, tokens, topk, vecs, runs,
-                                        reinterpret_cast<uint4*>(out), fp16);
-  MB200_CHECK_CUDA(cudaGetLastError());
-  return kOk;
+  return launch_chained(kernel, dim3(blocks), threads, 0, stream, false, chained, reinterpret_cast<const uint4*>(y),
+                        inverse, tokens, topk, vecs, runs, reinterpret_cast<uint4*>(out), fp16);
 }
 
 int launch_combine_push(const __nv_bfloat16* y, int all_tokens, int tokens_per_rank, int topk, int hidden,
@@ -236,16 +239,15 @@ int launch_sum_planes(const __nv_bfloat16* partial, int tokens, int world, int h
 }
 
 int launch_group_quant_fp8(const __nv_bfloat16* x, int64_t rows, int hidden, uint8_t* q, float* scales,
-                           int64_t scale_ld, int transposed, cudaStream_t stream, int ue8m0) {
+                           int64_t scale_ld, int transposed, cudaStream_t stream, int ue8m0, bool chained) {
   MB200_REQUIRE(hidden % 128 == 0, kUnsupportedShape, "group_quant: hidden=%d must be a multiple of 128", hidden);
   if (rows == 0) return kOk;
   const int threads = 256;
   const int blocks = grid_for(rows * (hidden / 128) * 8, threads, sm_count(), 16);
   auto kernel = ue8m0 ? group_quant_fp8_kernel<true> : group_quant_fp8_kernel<false>;
-  kernel<<<blocks, threads, 0, stream>>>(reinterpret_cast<const uint4*>(x), rows, hidden / 128,
-                                         reinterpret_cast<uint2*>(q), scales, scale_ld, transposed);
-  MB200_CHECK_CUDA(cudaGetLastError());
-  return kOk;
+  return launch_chained(kernel, dim3(blocks), threads, 0, stream, false, chained, reinterpret_cast<const uint4*>(x), rows,
+                        hidden / 128, reinterpret_cast<uint2*>(q), scales, scale_ld, transposed,
+                        int(chained));
 }
 
 }  // namespace mb200

@@ -1054,9 +1054,10 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         # kernels of this library launched per step (memsets and copies are not kernels); derived
         # from the call sequence of the entry points, checked against the committed ncu launch list
         total_assignments = assignments * world
-        n_align = 3 if total_assignments > 8192 else 1
-        if world == 1:      # align, [fp8: quantise + row gather], gate/up GEMM (16-bit: gather fused), down GEMM, combine
-            kernels_per_step = n_align + 3 + (2 if fp8 else 0)
+        align_experts = EXPERTS if world == 1 or leg.tp else EXPERTS // world
+        n_align = 2 if total_assignments > (4096 if align_experts <= 256 else 512) else 1
+        if world == 1:      # align, [fp8: quantise, few rows per expert: row gather], gate/up GEMM (gather fused), down GEMM, combine
+            kernels_per_step = n_align + 3 + (0 if not fp8 else 1 if disp["pad_rows"] == 128 else 2)
         else:
             kernels_per_step = _dist_kernels_per_step(n_align, fp8, leg.tp, not fp8 or disp["pad_rows"] == 128)
         line = {

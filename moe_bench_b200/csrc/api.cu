@@ -133,7 +133,7 @@ Layout make_layout(int precision, int64_t tokens, int hidden, int intermediate, 
   l.y = take((a > 0 ? a : 1) * int64_t(hidden) * 2);
   l.xs = l.acts = 0;
   // arrival counters per 16-row granule (fused dispatch) and completion counters per token
-  // block (fused combine push), adjacent so that one memset clears both
+  // block (fused combine push), adjacent so that one pass of the sort clears both
   l.granule_bytes = (cap / kPadBf16 + 1) * 4;
   l.granules = take(l.granule_bytes);
   l.block_bytes = (cap / kPadBf16 + 1) * 4;

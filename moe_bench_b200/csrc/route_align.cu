@@ -16,6 +16,7 @@
 //    blocks and experts, then a scatter that replays the same match.any ranks,
 //    so the order inside an expert is ascending n whatever the grid.
 
+#include "align_row.h"
 #include "layer.cuh"
 
 namespace mb200 {
@@ -296,9 +297,9 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
   }
   __syncthreads();
 
-  // 4. first row of every (warp, expert): expert's first row + blocks before + warps before
+  // 4. assignments of the expert ahead of every (warp, expert): blocks before + warps before
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = prefix[e] * pad + base[e];
+    int run = base[e];
     for (int w0 = 0; w0 < warps; w0 += 8) {  // 8 or 32 warps
       int v[8];
 #pragma unroll
@@ -319,16 +320,16 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
   // 5. place this warp's assignments; the experts' padding rows are shared out over all warps
   walk_chunk(topk_ids, expert_map, begin, end, E, [&](int64_t n, int slot, int before, unsigned peers) {
     if (slot < 0) { inverse[n] = -1; return; }
-    const int row = running[slot] + before;
+    const int64_t row = sorted_row(prefix[slot], pad, running[slot] + before);
     if (row < row_capacity) sorted_ids[row] = int(n);
-    inverse[n] = row;
+    inverse[n] = int(row);
     __syncwarp(peers);  // the peers have read the counter
     if (before == 0) running[slot] += __popc(peers);
   });
   for (int e = blockIdx.x * warps + warp; e < E; e += nb * warps) {
-    int64_t stop = int64_t(prefix[e + 1]) * pad;
+    int64_t stop = sorted_row(prefix[e + 1], pad, 0);
     if (stop > row_capacity) stop = row_capacity;
-    for (int64_t p = int64_t(prefix[e]) * pad + total[e] + lane; p < stop; p += 32) sorted_ids[p] = -1;
+    for (int64_t p = sorted_row(prefix[e], pad, total[e]) + lane; p < stop; p += 32) sorted_ids[p] = -1;
   }
 }
 

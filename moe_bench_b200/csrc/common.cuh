@@ -228,6 +228,9 @@ __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, Wa
 // still running (once all of that kernel's blocks have called pdl_trigger() or exited).
 // pdl_wait() returns when the kernels before it have completed and their writes are visible;
 // every such kernel calls it before it exits, so completion stays transitive along the stream.
+// Such a kernel reads what a kernel ahead of it may still be writing with coherent loads (__ldcg,
+// plain), through pointers that are not `const __restrict__`: a read-only-cache load promises data
+// that is constant for the kernel's lifetime, and the compiler may move it across the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

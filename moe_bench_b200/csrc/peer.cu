@@ -98,20 +98,19 @@ __global__ void gather_blocks_peer_kernel(PeerTable src, int rank, int world, in
 // Sorted rows pulled from the source ranks.  n = (ring*T + t)*k + j.
 // e4m3 rows + their scales ([T][K/128] at the source) -> sorted rows + group-major scales.
 __global__ void gather_rows_peer_fp8_kernel(PeerTable xq, PeerTable xs, int rank, int world, int tokens,
-                                            int topk, const int* __restrict__ sorted_ids,
-                                            const int* __restrict__ mtile_prefix, int local_experts,
+                                            int topk, const int* sorted_ids, const int* mtile_prefix, int local_experts,
                                             int groups_per_row, uint4* __restrict__ out_q,
                                             float* __restrict__ out_scales_t, int64_t row_capacity, int pad) {
   pdl_wait();
   pdl_trigger();  // after the wait: the kernel that follows may rely on the schedule
-  int64_t rows = int64_t(__ldg(mtile_prefix + local_experts)) * pad;
+  int64_t rows = int64_t(__ldcg(mtile_prefix + local_experts)) * pad;
   if (rows > row_capacity) rows = row_capacity;
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int vec_per_row = groups_per_row * 8;  // 128 bytes per group = 8 x 16 bytes
   for (int64_t row = int64_t(blockIdx.x) * warps_per_block + (threadIdx.x >> 5); row < rows;
        row += int64_t(gridDim.x) * warps_per_block) {
-    const int n = __ldg(sorted_ids + row);
+    const int n = __ldcg(sorted_ids + row);
     if (n < 0) continue;
     const int tok_global = n / topk;
     const int ring = tok_global / tokens;

@@ -196,7 +196,7 @@ __global__ void align_count_kernel(const int* __restrict__ topk_ids, const int* 
 // Shared memory, ints: per_warp [warps][E] | total [E] | base [E] | prefix [E+1] | part [2][threads]
 __global__ void __launch_bounds__(kMaxAlignWarps * 32)
 align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ expert_map, int64_t assignments,
-                     int local_experts, int64_t chunk, const int* __restrict__ block_hist,
+                     int local_experts, int64_t chunk, const int* block_hist,
                      int* __restrict__ counts, int* __restrict__ mtile_prefix, int* __restrict__ sorted_ids,
                      int* __restrict__ inverse, int64_t row_capacity, int pad, int* __restrict__ clear,
                      int64_t clear_ints) {
@@ -244,7 +244,7 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int r = r0 + i * groups;
-          v[i] = r >= rows ? 0 : nb > 1 ? __ldg(block_hist + size_t(r) * E + e) : per_warp[r * E + e];
+          v[i] = r >= rows ? 0 : nb > 1 ? __ldcg(block_hist + size_t(r) * E + e) : per_warp[r * E + e];
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {

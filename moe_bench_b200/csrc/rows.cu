@@ -27,7 +27,7 @@ namespace {
 // <1, 8> for fewer tokens: all rows of a vector in one round trip, on four times the warps.
 template <int kVecs, int kRows>
 __global__ void __launch_bounds__(256)
-combine_bf16_kernel(const uint4* __restrict__ y, const int* __restrict__ inverse, int tokens, int topk,
+combine_bf16_kernel(const uint4* y, const int* inverse, int tokens, int topk,
                     int vec_per_row, int runs, uint4* __restrict__ out, int fp16) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -45,7 +45,7 @@ combine_bf16_kernel(const uint4* __restrict__ y, const int* __restrict__ inverse
       const int j = j0 + lane;
       // an expert on another rank contributes zero
       unsigned present =
-          __ballot_sync(0xffffffffu, j < topk && (inverse == nullptr || __ldg(inverse + t * topk + j) >= 0));
+          __ballot_sync(0xffffffffu, j < topk && (inverse == nullptr || __ldcg(inverse + t * topk + j) >= 0));
       while (present) {  // summed in ascending j
         uint4 val[kRows][kVecs];
         const int n = min(__popc(present), kRows);
@@ -57,7 +57,7 @@ combine_bf16_kernel(const uint4* __restrict__ y, const int* __restrict__ inverse
             const uint4* row = y + (t * topk + jj) * vec_per_row;
 #pragma unroll
             for (int c = 0; c < kVecs; ++c)
-              if (v0 + 32 * c < vec_per_row) val[u][c] = __ldg(row + v0 + 32 * c);
+              if (v0 + 32 * c < vec_per_row) val[u][c] = __ldcg(row + v0 + 32 * c);
           }
         }
 #pragma unroll

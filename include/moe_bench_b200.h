@@ -43,7 +43,10 @@ int mb200_abi_version(void);
 const char* mb200_last_error(void);
 
 /* Router front end: softmax over `experts` logits, top-k (largest first, lowest
- * index wins ties), weights renormalised over the selection.
+ * index wins ties), weights renormalised over the selection.  The ids of a row are
+ * topk different experts whatever its logits are: -inf comes after every finite
+ * logit and NaN after -inf, both with weight 0; a row with no finite logit, or with
+ * +inf, gets its ids by the same order and NaN weights, as softmax gives.
  * logits [tokens, experts] fp32 -> topk_ids [tokens, topk] int32,
  * topk_weights [tokens, topk] fp32.  The reference has no router: it draws ids
  * and weights directly (data.py:178-235). */

@@ -26,18 +26,20 @@ namespace {
 // ---------------------------------------------------------------- route_topk
 constexpr int kRouteMaxExperts = 1024;
 
-// Order-preserving image of a logit in uint32: larger logit <-> larger key, -0 == +0.
-// NaN maps to 0, below the key of -inf: a NaN logit is never selected.
+// Order-preserving image of a logit in uint32: larger logit <-> larger key, -0 == +0, NaN below
+// -inf, and 0 below all of them for what cannot be selected (an earlier winner, a slot past the last
+// expert).  Every expert of the row has a key above 0 until it is selected, so topk <= experts rounds
+// give topk different experts, whatever the logits are.
+constexpr uint32_t kKeyNone = 0u, kKeyNan = 1u;  // logit_key(-inf) = 0x007FFFFF
 __device__ __forceinline__ uint32_t logit_key(float v) {
   const uint32_t u = __float_as_uint(v + 0.0f);  // -0 + 0 = +0
   const uint32_t key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-  return v != v ? 0u : key;
+  return v != v ? kKeyNan : key;
 }
 __device__ __forceinline__ float key_logit(uint32_t key) {
-  if (key == 0u) return -INFINITY;  // nothing but NaN in the row
+  if (key <= kKeyNan) return -INFINITY;  // a NaN logit weighs nothing beside others
   return __uint_as_float((key & 0x80000000u) ? (key ^ 0x80000000u) : ~key);
 }
-constexpr uint32_t kKeyNegInf = 0x007FFFFFu;  // logit_key(-inf)
 
 // One warp per token, lane l holds experts l, l+32, ... (coalesced loads) as ordered integer
 // keys.  Instruction issue bounds this kernel (the 8 MB of logits are two microseconds of HBM), so
@@ -59,12 +61,12 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, 
 #pragma unroll
   for (int i = 0; i < kPerLane; ++i) {
     const int e = i * 32 + lane;
-    key[i] = e < experts ? logit_key(__ldg(row + e)) : 0u;
+    key[i] = e < experts ? logit_key(__ldg(row + e)) : kKeyNone;
   }
   uint32_t best;
   int best_e;
   auto rescan = [&]() {  // lowest index first on ties (i ascending, strict >)
-    best = 0u;
+    best = kKeyNone;
     best_e = 0x7fffffff;
 #pragma unroll
     for (int i = 0; i < kPerLane; ++i)
@@ -81,11 +83,11 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, 
     const int win_e = __reduce_min_sync(0xffffffffu, best == win ? best_e : 0x7fffffff);
     if (j == 0) mx = key_logit(win);
     if (lane == (j & 31)) { my_key = win; my_id = win_e; }
-    // retire the winner (as -inf, like an expert masked by the caller)
+    // retire the winner
     if (best_e == win_e) {
 #pragma unroll
       for (int i = 0; i < kPerLane; ++i)
-        if (i * 32 + lane == win_e) key[i] = kKeyNegInf;
+        if (i * 32 + lane == win_e) key[i] = kKeyNone;
       rescan();
     }
     if ((j & 31) == 31 || j == topk - 1) {

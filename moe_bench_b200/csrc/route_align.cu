@@ -153,7 +153,8 @@ __device__ __forceinline__ int slot_of(const int* topk_ids, const int* expert_ma
 
 // Walk one chunk in order, 32 assignments at a time (the loads of four steps in flight
 // together).  Emit(n, slot, before, peers): `peers` are the lanes with the same slot, `before`
-// how many of them come first; called by every lane whose assignment exists.
+// how many of them come first; called by the whole warp, converged (slot -1 and n >= end where a lane
+// has no assignment).
 template <class Emit>
 __device__ __forceinline__ void walk_chunk(const int* topk_ids, const int* expert_map, int64_t begin,
                                            int64_t end, int local_experts, Emit emit) {
@@ -171,7 +172,7 @@ __device__ __forceinline__ void walk_chunk(const int* topk_ids, const int* exper
       if (base + 32 * i >= end) break;
       const int64_t n = base + 32 * i + lane;
       const unsigned peers = __match_any_sync(0xffffffffu, slot[i]);
-      if (n < end) emit(n, slot[i], __popc(peers & ((1u << lane) - 1u)), peers);
+      emit(n, slot[i], __popc(peers & ((1u << lane) - 1u)), peers);
       __syncwarp();
     }
   }
@@ -321,12 +322,19 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
 
   // 5. place this warp's assignments; the experts' padding rows are shared out over all warps
   walk_chunk(topk_ids, expert_map, begin, end, E, [&](int64_t n, int slot, int before, unsigned peers) {
-    if (slot < 0) { inverse[n] = -1; return; }
-    const int64_t row = sorted_row(prefix[slot], pad, running[slot] + before);
-    if (row < row_capacity) sorted_ids[row] = int(n);
-    inverse[n] = int(row);
-    __syncwarp(peers);  // the peers have read the counter
-    if (before == 0) running[slot] += __popc(peers);
+    const int seen = slot >= 0 ? running[slot] : 0;
+    // All lanes have read their counters.  One barrier for the warp: with one per group of peers the
+    // groups, up to 32, run one after the other (4096 assignments over 256 experts in one block: 23.0
+    // against 18.8 us).
+    __syncwarp();
+    if (slot >= 0) {
+      const int64_t row = sorted_row(prefix[slot], pad, seen + before);
+      if (row < row_capacity) sorted_ids[row] = int(n);
+      inverse[n] = int(row);
+      if (before == 0) running[slot] = seen + __popc(peers);
+    } else if (n < end) {
+      inverse[n] = -1;
+    }
   });
   for (int e = blockIdx.x * warps + warp; e < E; e += nb * warps) {
     int64_t stop = sorted_row(prefix[e + 1], pad, 0);

@@ -1054,8 +1054,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         # kernels of this library launched per step (memsets and copies are not kernels); derived
         # from the call sequence of the entry points, checked against the committed ncu launch list
         total_assignments = assignments * world
-        align_experts = EXPERTS if world == 1 or leg.tp else EXPERTS // world
-        n_align = 2 if total_assignments > (4096 if align_experts <= 256 else 512) else 1
+        n_align = 2 if total_assignments > 1024 else 1
         if world == 1:      # align, [fp8: quantise, few rows per expert: row gather], gate/up GEMM (gather fused), down GEMM, combine
             kernels_per_step = n_align + 3 + (0 if not fp8 else 1 if disp["pad_rows"] == 128 else 2)
         else:

@@ -118,28 +118,31 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, 
 // block redoing the (small) scans for itself, so no single-block pass sits between the two.  One
 // block needs no histogram but its own: up to kOneBlockAssignments a single launch does it all.
 // The work is latency, not bandwidth (8192 tokens x top-8: 0.8 MB): chunks are short, so that many
-// warps wait at the same time, and everything a block shares stays in shared memory.  Measured
-// between stage events (launch gaps included): 8192 tokens, 256 experts 44 -> 32 us; 32768 tokens,
-// 32 local experts 31 -> 21 us; against count, one-block scan and scatter as three kernels, with the
-// arrival counters of the GEMMs cleared by a memset of their own.
+// warps wait at the same time, and everything a block shares stays in shared memory.  16 warps of at
+// least 32 assignments, at every size: fewer warps leave more histograms for every block to sum and
+// fewer threads to sum them (65536 assignments over 1024 experts: 8 warps 58.9 us, 16 warps 40.7; count,
+// one-block scan and scatter as three kernels 42.0), more warps or longer chunks lengthen the walks of
+// one block (4096 over 256: 32 warps of 128 in one block 18.8 us, 16 warps of 32 in 8 blocks 8.9).
+// Device time of a call, one B200, the three kernels against these two: 512 over 256 experts 10.4 / 10.2
+// us, 8192 over 256 27.7 / 9.1, 65536 over 256 25.2 / 14.8, 524288 over 32 25.8 / 17.7.
 constexpr int kMaxUnits = 1024;            // scratch: this many ints per expert
-constexpr int kMaxAlignWarps = 32;
-constexpr int kMinChunk = 64;              // assignments per warp
-constexpr int kOneBlockAssignments = 4096;
+constexpr int kAlignWarps = 16;            // per block
+constexpr int kMinChunk = 32;              // assignments per warp
+// Above a block of shortest chunks, because a second launch costs what it saves: 1024 assignments over 8
+// experts 5.7 us in one block, 6.8 in two (over 256 experts 11.8 and 10.3).
+constexpr int kOneBlockAssignments = 1024;
 
 struct AlignShape {
-  int warps;   // per block: the per-warp counters of a block fit 48 KiB of shared memory
   int blocks;
   int64_t chunk;
 };
-AlignShape align_shape(int64_t assignments, int experts) {
+AlignShape align_shape(int64_t assignments) {
   AlignShape s;
-  s.warps = experts <= 256 ? kMaxAlignWarps : 8;
-  const int64_t max_blocks = assignments <= kOneBlockAssignments && s.warps == kMaxAlignWarps ? 1 : kMaxUnits / 4;
-  int64_t chunk = (assignments + max_blocks * s.warps - 1) / (max_blocks * s.warps);
-  chunk = (chunk + 31) / 32 * 32;
+  constexpr int64_t kMaxWarps = int64_t(kMaxUnits / 4) * kAlignWarps;  // of the whole grid
+  const int64_t warps = assignments <= kOneBlockAssignments ? kAlignWarps : kMaxWarps;
+  const int64_t chunk = ((assignments + warps - 1) / warps + 31) / 32 * 32;
   s.chunk = chunk < kMinChunk ? kMinChunk : chunk;
-  const int64_t per_block = s.chunk * s.warps;
+  const int64_t per_block = s.chunk * kAlignWarps;
   s.blocks = assignments <= per_block ? 1 : int((assignments + per_block - 1) / per_block);
   return s;
 }
@@ -197,7 +200,7 @@ __global__ void align_count_kernel(const int* __restrict__ topk_ids, const int* 
 }
 
 // Shared memory, ints: per_warp [warps][E] | total [E] | base [E] | prefix [E+1] | part [2][threads]
-__global__ void __launch_bounds__(kMaxAlignWarps * 32)
+__global__ void __launch_bounds__(kAlignWarps * 32)
 align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ expert_map, int64_t assignments,
                      int local_experts, int64_t chunk, const int* block_hist,
                      int* __restrict__ counts, int* __restrict__ mtile_prefix, int* __restrict__ sorted_ids,
@@ -205,7 +208,9 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
                      int64_t clear_ints) {
   extern __shared__ int smem[];
   const int E = local_experts;
-  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int warps = kAlignWarps;
+  static_assert(kAlignWarps % 8 == 0, "the warps' counters are read eight at a time");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* per_warp = smem;
   int* total = per_warp + warps * E;
   int* base = total + E;
@@ -303,7 +308,7 @@ align_scatter_kernel(const int* __restrict__ topk_ids, const int* __restrict__ e
   // 4. assignments of the expert ahead of every (warp, expert): blocks before + warps before
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     int run = base[e];
-    for (int w0 = 0; w0 < warps; w0 += 8) {  // 8 or 32 warps
+    for (int w0 = 0; w0 < warps; w0 += 8) {
       int v[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = per_warp[(w0 + i) * E + e];
@@ -382,14 +387,18 @@ int launch_align(const int* topk_ids, int64_t assignments, const int* expert_map
                 "align: %lld assignments do not fit 32-bit row indices", (long long)assignments);
   const int pad = sched.pad_rows;
   MB200_REQUIRE(pad >= 1 && pad <= 1024, kInvalidArgument, "align: pad_rows=%d (1..1024)", pad);
-  const AlignShape sh = align_shape(assignments, local_experts);
-  const int threads = sh.warps * 32;
+  const AlignShape sh = align_shape(assignments);
+  constexpr int threads = kAlignWarps * 32;
   if (sh.blocks > 1) {
     align_count_kernel<<<sh.blocks, threads, size_t(local_experts) * sizeof(int), stream>>>(
         topk_ids, expert_map, assignments, local_experts, sh.chunk, scratch);
     MB200_CHECK_CUDA(cudaGetLastError());
   }
-  const size_t smem = size_t(sh.warps * local_experts + 3 * local_experts + 1 + 2 * threads) * sizeof(int);
+  auto smem_bytes = [](int experts) { return size_t(kAlignWarps * experts + 3 * experts + 1 + 2 * threads) * sizeof(int); };
+  const size_t smem = smem_bytes(local_experts);
+  if (smem > 48 * 1024)  // more than 592 experts
+    MB200_CHECK_CUDA(cudaFuncSetAttribute(align_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          int(smem_bytes(kMaxExperts))));
   // The first kernel of the sort is an ordinary launch: what came before it on the stream is
   // complete, so the second may overlap the first up to the histograms.
   if (sh.blocks > 1)

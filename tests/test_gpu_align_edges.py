@@ -1,5 +1,5 @@
-"""Sort-and-pad where its launch shape changes: one block
-or several (4096 assignments; 512 beyond 256 experts), longer chunks (2^19 and 2^17)."""
+"""Sort-and-pad where its launch shape changes: one block or several (1024 assignments), longer chunks
+(2^17), more than 48 KiB of shared memory (592 experts); and runs of one expert or none in a warp."""
 
 import numpy as np
 import pytest
@@ -14,7 +14,8 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("assignments,experts", [(1, 1), (512, 256), (513, 256), (1024, 7), (1025, 256), (4096, 256),
                                                  (4097, 256), (512, 257), (513, 257), (131072, 300), (131073, 300),
-                                                 (524289, 32)])
+                                                 (524289, 32), (131072, 32), (131073, 32), (1000, 592), (1000, 593),
+                                                 (65537, 1024), (1024, 256), (1025, 1), (2049, 2)])
 @pytest.mark.parametrize("mapped", [False, True])
 def test_align_at_the_edges(assignments, experts, mapped):
     rng = np.random.default_rng(assignments + experts)

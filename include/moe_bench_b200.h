@@ -78,8 +78,8 @@ int mb200_align(const int32_t* topk_ids, int64_t tokens, int topk, const int32_t
  * Who needs it: a serving process that gave all of HBM to its own memory pool
  * at start-up cannot get a scratch buffer from cudaMalloc later, and a decode
  * loop with a latency budget cannot afford the device-wide stall a
- * cudaMalloc/cudaFree causes.  Here the sort's scratch (per-unit expert
- * histograms) is a fixed 1 MiB array inside the library, so the caller passes
+ * cudaMalloc/cudaFree causes.  Here the sort's scratch (per-block expert
+ * histograms) is a fixed 256 KiB array inside the library, so the caller passes
  * only inputs and outputs and the call allocates nothing (no cudaMalloc,
  * cudaFree or allocating library routine).
  *
@@ -87,7 +87,7 @@ int mb200_align(const int32_t* topk_ids, int64_t tokens, int topk, const int32_t
  *  - local_experts <= MB200_NOALLOC_MAX_LOCAL_EXPERTS and tokens*topk <=
  *    MB200_NOALLOC_MAX_ASSIGNMENTS; larger problems are refused with status 5
  *    and a message naming mb200_align as the alternative;
- *  - every GPU that loads the library holds the 1 MiB array until the process
+ *  - every GPU that loads the library holds the 256 KiB array until the process
  *    exits, whether or not this entry point is used;
  *  - the first call on a device looks up the array's device address
  *    (cudaGetSymbolAddress, with that device current); make that first call

@@ -230,7 +230,7 @@ def align_noalloc(topk_ids: torch.Tensor, expert_map: Optional[torch.Tensor], lo
 
     For hosts that may not allocate device memory while running (a server
     whose pool owns all of HBM, a latency-bound decode loop): the library's
-    built-in 1 MiB array replaces the scratch tensor.  Pass ``outputs`` =
+    built-in 256 KiB array replaces the scratch tensor.  Pass ``outputs`` =
     ``(counts, mtile_prefix, sorted_ids, inverse)`` preallocated to make the
     whole call allocation-free; without it the four output tensors are created
     here for convenience.  Limits: 256 local experts, 2**20 assignments; calls

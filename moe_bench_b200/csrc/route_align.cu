@@ -125,7 +125,7 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int tokens, 
 // one block (4096 over 256: 32 warps of 128 in one block 18.8 us, 16 warps of 32 in 8 blocks 8.9).
 // Device time of a call, one B200, the three kernels against these two: 512 over 256 experts 10.4 / 10.2
 // us, 8192 over 256 27.7 / 9.1, 65536 over 256 25.2 / 14.8, 524288 over 32 25.8 / 17.7.
-constexpr int kMaxUnits = 1024;            // scratch: this many ints per expert
+constexpr int kMaxAlignBlocks = 256;       // one histogram each: scratch is this many ints per expert
 constexpr int kAlignWarps = 16;            // per block
 constexpr int kMinChunk = 32;              // assignments per warp
 // Above a block of shortest chunks, because a second launch costs what it saves: 1024 assignments over 8
@@ -138,7 +138,7 @@ struct AlignShape {
 };
 AlignShape align_shape(int64_t assignments) {
   AlignShape s;
-  constexpr int64_t kMaxWarps = int64_t(kMaxUnits / 4) * kAlignWarps;  // of the whole grid
+  constexpr int64_t kMaxWarps = int64_t(kMaxAlignBlocks) * kAlignWarps;  // of the whole grid
   const int64_t warps = assignments <= kOneBlockAssignments ? kAlignWarps : kMaxWarps;
   const int64_t chunk = ((assignments + warps - 1) / warps + 31) / 32 * 32;
   s.chunk = chunk < kMinChunk ? kMinChunk : chunk;
@@ -374,9 +374,8 @@ int launch_route_topk(const float* logits, int tokens, int experts, int topk, in
 }
 
 int64_t align_scratch_ints(int64_t assignments, int experts) {
-  int64_t units = kMaxUnits;
   (void)assignments;
-  return units * experts;
+  return int64_t(kMaxAlignBlocks) * experts;
 }
 
 int launch_align(const int* topk_ids, int64_t assignments, const int* expert_map, int local_experts,
@@ -421,8 +420,8 @@ int launch_align(const int* topk_ids, int64_t assignments, const int* expert_map
 // running: an inference server that handed (nearly) all HBM to its own pool at
 // start-up has nothing left for a later cudaMalloc, and inside a latency-
 // critical decode loop cudaMalloc/cudaFree would stall the whole device.  For
-// them the unit histograms of the sort live in the fixed array below instead of
-// a buffer the caller allocates.  The price: 1 MiB of every GPU that loads the
+// them the blocks' histograms of the sort live in the fixed array below instead of
+// a buffer the caller allocates.  The price: 256 KiB of every GPU that loads the
 // library is held until the process exits, the problem size is capped, and all
 // calls on a device share the one array.
 // ---------------------------------------------------------------------------
@@ -435,8 +434,8 @@ namespace {
 
 constexpr int kNoAllocMaxExperts = MB200_NOALLOC_MAX_LOCAL_EXPERTS;          // 256
 constexpr int64_t kNoAllocMaxAssignments = MB200_NOALLOC_MAX_ASSIGNMENTS;    // 2^20
-// units (<= 1024) x experts (<= 256) histogram entries = 1 MiB
-static __device__ __align__(256) int g_noalloc_align_scratch[kMaxUnits * kNoAllocMaxExperts];
+// blocks (<= 256) x experts (<= 256) histogram entries = 256 KiB
+static __device__ __align__(256) int g_noalloc_align_scratch[kMaxAlignBlocks * kNoAllocMaxExperts];
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mutex;

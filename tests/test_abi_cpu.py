@@ -48,6 +48,12 @@ def test_abi_version_and_pure_host_queries(lib):
     assert lib.mb200_workspace_bytes(capi.PRECISION_FP16, 128, 7168, 2048, 256, 8) == n
 
 
+@pytest.mark.parametrize("tokens,topk,experts", [(0, 8, 256), (1, 1, 1), (8192, 8, 256), (1 << 20, 8, 1024)])
+def test_sort_scratch_is_what_the_sort_can_use(lib, tokens, topk, experts):
+    # one histogram of 4-byte counters for each of at most 256 blocks
+    assert lib.mb200_align_scratch_bytes(tokens, topk, experts) == 256 * experts * 4
+
+
 def test_argument_errors_are_reported_not_fatal(lib):
     assert lib.mb200_workspace_bytes(capi.PRECISION_BF16, 4, 100, 128, 8, 2) == -1
     assert b"hidden" in lib.mb200_last_error()

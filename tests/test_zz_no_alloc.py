@@ -40,7 +40,7 @@ def _same(a, b):
 
 
 def test_noalloc_align_matches_align_on_consecutive_calls():
-    # 1) large: three-kernel path, fills many unit histograms of the shared array
+    # 1) large: two-kernel path, fills many block histograms of the shared array
     # 2) small, fewer experts: one-block path, reads a different part of the same array
     # 3) expert-parallel map with empty experts, again after a larger call
     cases = [

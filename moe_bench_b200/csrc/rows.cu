@@ -18,34 +18,40 @@ namespace mb200 {
 
 namespace {
 
-// One warp per (token, run of 32*kVecs vectors).  The lanes read the token's k entries of
-// `inverse` once and ballot them, so the warp walks only the assignments that are present, kRows
-// rows x kVecs vectors of a lane in flight whatever their number.  (With one vector per thread and
+// One group of kLanes lanes per (token, run of kLanes*kVecs vectors).  The lanes read the token's k
+// entries of `inverse` once and ballot them, so the group walks only the assignments that are present,
+// kRows rows x kVecs vectors of a lane in flight whatever their number.  (With one vector per thread and
 // a test of `inverse` before each of k loads, a rank of 8, which holds about one row per token,
-// had that one load in flight: 32768 tokens 471 us, now 207 of the 141 that its 0.94 GB take;
-// all rows local, 8192 tokens 214 -> 173 us, 1.06 GB at 6.1 TB/s.)  <4, 4> once it fills the GPU,
-// <1, 8> for fewer tokens: all rows of a vector in one round trip, on four times the warps.
-template <int kVecs, int kRows>
+// had that one load in flight: 32768 tokens 435 us, now 195 of the 141 that its 0.94 GB take;
+// all rows local, 8192 tokens 181 -> 157 us, 1.06 GB at 6.7 TB/s.)  Narrow rows need narrow groups, or
+// most lanes have no vector: 32768 tokens x 8 rows of 64 / 576 / 1152 elements 38.8 / 68.8 / 130.0 us
+// with whole warps, 7.6 / 60.8 / 108.9 in groups of 8 (one vector per thread: 8.1 / 63.8 / 120.7).
+template <int kLanes, int kVecs, int kRows>
 __global__ void __launch_bounds__(256)
 combine_bf16_kernel(const uint4* y, const int* inverse, int tokens, int topk,
                     int vec_per_row, int runs, uint4* __restrict__ out, int fp16) {
   pdl_wait();
-  const int lane = threadIdx.x & 31;
+  constexpr int kGroups = 32 / kLanes;  // runs a warp works on side by side
+  const int lane = threadIdx.x & (kLanes - 1), group = (threadIdx.x & 31) / kLanes;
   const int64_t total = int64_t(tokens) * runs;
-  for (int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; i < total;
-       i += (int64_t(gridDim.x) * blockDim.x) >> 5) {
-    const int64_t t = i / runs;
-    const int v0 = int(i - t * runs) * 32 * kVecs + lane;
+  // the loops up to the ballot have the same trip count in the whole warp
+  for (int64_t first = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups; first < total;
+       first += ((int64_t(gridDim.x) * blockDim.x) >> 5) * kGroups) {
+    const int64_t i = first + group;
+    const bool active = i < total;
+    const int64_t t = active ? i / runs : 0;
+    const int v0 = active ? int(i - t * runs) * kLanes * kVecs + lane : vec_per_row;
     float acc[kVecs][8];
 #pragma unroll
     for (int c = 0; c < kVecs; ++c)
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc[c][k] = 0.f;
-    for (int j0 = 0; j0 < topk; j0 += 32) {
+    for (int j0 = 0; j0 < topk; j0 += kLanes) {
       const int j = j0 + lane;
       // an expert on another rank contributes zero
-      unsigned present =
-          __ballot_sync(0xffffffffu, j < topk && (inverse == nullptr || __ldcg(inverse + t * topk + j) >= 0));
+      unsigned present = __ballot_sync(
+          0xffffffffu, active && j < topk && (inverse == nullptr || __ldcg(inverse + t * topk + j) >= 0));
+      if (kLanes < 32) present = (present >> (group * kLanes)) & ((1u << (kLanes & 31)) - 1u);
       while (present) {  // summed in ascending j
         uint4 val[kRows][kVecs];
         const int n = min(__popc(present), kRows);
@@ -57,7 +63,7 @@ combine_bf16_kernel(const uint4* y, const int* inverse, int tokens, int topk,
             const uint4* row = y + (t * topk + jj) * vec_per_row;
 #pragma unroll
             for (int c = 0; c < kVecs; ++c)
-              if (v0 + 32 * c < vec_per_row) val[u][c] = __ldcg(row + v0 + 32 * c);
+              if (v0 + kLanes * c < vec_per_row) val[u][c] = __ldcg(row + v0 + kLanes * c);
           }
         }
 #pragma unroll
@@ -65,12 +71,12 @@ combine_bf16_kernel(const uint4* y, const int* inverse, int tokens, int topk,
           if (u < n)
 #pragma unroll
             for (int c = 0; c < kVecs; ++c)
-              if (v0 + 32 * c < vec_per_row) add_h16x8(val[u][c], acc[c], fp16);
+              if (v0 + kLanes * c < vec_per_row) add_h16x8(val[u][c], acc[c], fp16);
       }
     }
 #pragma unroll
     for (int c = 0; c < kVecs; ++c)
-      if (v0 + 32 * c < vec_per_row) out[t * vec_per_row + v0 + 32 * c] = pack_h16x8(acc[c], fp16);
+      if (v0 + kLanes * c < vec_per_row) out[t * vec_per_row + v0 + kLanes * c] = pack_h16x8(acc[c], fp16);
   }
 }
 
@@ -209,10 +215,22 @@ int launch_combine_bf16(const __nv_bfloat16* y, const int* inverse, int tokens, 
   if (tokens == 0) return kOk;
   const int threads = 256, sms = sm_count();
   const int vecs = hidden / 8;
-  const bool wide = int64_t(tokens) * ((vecs + 127) / 128) >= int64_t(sms) * 16;  // a warp per run, 16 warps per SM
-  const int runs = wide ? (vecs + 127) / 128 : (vecs + 31) / 32;
-  const int blocks = grid_for(int64_t(tokens) * runs * 32, threads, sms, 16);
-  auto kernel = wide ? combine_bf16_kernel<4, 4> : combine_bf16_kernel<1, 8>;
+  // Whole rows of 128 vectors keep every lane of a warp and all its loads busy; rows that leave a
+  // quarter of them idle go to groups of 8 lanes (hidden is a multiple of 64 in every layer, so 8
+  // lanes always come out even).  Few tokens: one round trip on as many warps as there are.
+  const int sweep = (vecs + 127) / 128;
+  const bool fills = int64_t(tokens) * sweep >= int64_t(sms) * 16;  // a warp per run, 16 warps per SM
+  auto kernel = combine_bf16_kernel<32, 1, 8>;
+  int lanes = 32, per_run = 32;
+  if (fills && vecs * 8 >= sweep * 128 * 7) {
+    kernel = combine_bf16_kernel<32, 4, 4>, per_run = 128;
+  } else if (fills && vecs >= 64) {
+    kernel = combine_bf16_kernel<8, 2, 4>, lanes = 8, per_run = 16;
+  } else if (fills) {
+    kernel = combine_bf16_kernel<8, 1, 8>, lanes = 8, per_run = 8;
+  }
+  const int runs = (vecs + per_run - 1) / per_run;
+  const int blocks = grid_for(int64_t(tokens) * runs * lanes, threads, sms, 16);
   return launch_chained(kernel, dim3(blocks), threads, 0, stream, false, chained, reinterpret_cast<const uint4*>(y),
                         inverse, tokens, topk, vecs, runs, reinterpret_cast<uint4*>(out), fp16);
 }

@@ -1,7 +1,7 @@
 """16-bit layer where its kernels change shape: short K in the down GEMM with one accumulator pair
 (segments past 128 rows; fewer K steps than pipeline stages), ragged feature blocks, single and many
-experts, and both forms of the combine (few tokens / enough to fill the GPU), all rows local or one
-rank's share of them."""
+experts, and all forms of the combine (few tokens / enough to fill the GPU, wide / narrow rows), all
+rows local or one rank's share of them."""
 
 import pytest
 import torch
@@ -19,9 +19,14 @@ CASES = [
     (300, 576, 128, 4, 2, "uniform", "tp", 1),     # two K steps, ragged last 256-feature block
     (1100, 512, 192, 8, 3, "skewed", "tp", 1),     # segments of 50 to 1000 rows, three K steps
     (700, 768, 256, 5, 2, "single", "tp", 1),      # four K steps, more than the ring holds; empty experts
-    (2400, 320, 64, 8, 5, "uniform", "ep", 4),     # wide combine, a quarter of the rows local
-    (2367, 64, 64, 40, 9, "balanced", "tp", 1),    # narrow combine, k > 8, 8 vectors per row
+    (2400, 320, 64, 8, 5, "uniform", "ep", 4),     # narrow groups, a quarter of the rows local
+    (2367, 64, 64, 40, 9, "balanced", "tp", 1),    # too few tokens for narrow groups, k > 8, 8 vectors per row
     (40, 2048, 512, 640, 8, "uniform", "tp", 1),   # tile lookup over more experts than 32 x 16
+    (2368, 64, 64, 40, 9, "balanced", "tp", 1),    # combine in groups of 8 lanes, one vector each; k > 8
+    (2367, 192, 64, 16, 3, "uniform", "ep", 2),    # the last size of whole warps for rows that do not fill them
+    (2371, 576, 64, 8, 5, "uniform", "ep", 4),     # two vectors a lane, ragged last run, absent rows
+    (1187, 1152, 64, 24, 17, "uniform", "tp", 1),  # the same over two sweeps of 128, k > 16
+    (2368, 896, 64, 8, 2, "uniform", "tp", 1),     # whole warps, the last quarter of the lanes' vectors half empty
 ]
 
 

@@ -67,7 +67,8 @@ int64_t mb200_align_scratch_bytes(int64_t tokens, int topk, int local_experts);
  * counts [E], mtile_prefix [E+1] (cumulative pad_rows-row blocks; padded row offset
  * of expert e is pad_rows*mtile_prefix[e]), sorted_ids [row_capacity] (flat assignment
  * index token*topk+kpos per row, -1 for padding), inverse [tokens*topk] (row of
- * each assignment, -1 if its expert is not local). */
+ * each assignment, -1 if its expert is not local).  Up to 2^31 - 4097 assignments; sorted_ids is
+ * right for all of them, inverse holds the low 32 bits of a row past 2^31 - 1. */
 int mb200_align(const int32_t* topk_ids, int64_t tokens, int topk, const int32_t* expert_map,
                 int local_experts, int32_t* counts, int32_t* mtile_prefix, int32_t* sorted_ids,
                 int32_t* inverse, int64_t row_capacity, int pad_rows, void* scratch, void* stream);

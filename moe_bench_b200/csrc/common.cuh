@@ -112,7 +112,7 @@ __device__ __forceinline__ float fp8_group_scale(float amax, int ue8m0) {
 }
 
 // x / scale clamped to the e4m3 range, as the quantisers round it.  A power-of-two scale divides
-// exactly, and so does multiplying by its reciprocal (also exact: 2^-41 <= scale <= 2^120, or
+// exactly, and so does multiplying by its reciprocal (also exact: 2^-33 <= scale <= 2^120, or
 // inf -> 0): both round the same real number, so the bytes are the same as the division's
 // without its ~10 instructions per element.
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }

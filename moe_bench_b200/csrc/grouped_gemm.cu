@@ -23,10 +23,12 @@
 // One persistent CTA per SM, 512 threads: warp 0 issues TMA loads into a ring of
 // 128-byte-swizzled stages (32 KiB of weights + exactly the tile's token rows, one
 // TMA box per set bit of ntok/16), warp 1 owns tensor memory and issues tcgen05.mma,
-// warps 2-9 drain the accumulators: tcgen05.ld of two 16-token chunks per round
-// trip, accumulator released after the warp's last load, each chunk rounded,
-// transposed through a 1 KiB per-warp block of shared memory and stored as 16-byte
-// vectors (8 features of one token per thread).  Warps 10-13 are the fused dispatch
+// warps 2-9 drain the accumulators: tcgen05.ld of several chunks of 32 features x
+// 16 tokens per round trip, as fragments of 8x8 matrices, each chunk rounded,
+// transposed by stmatrix through a 1 KiB per-warp block of shared memory and stored
+// as 16-byte vectors (8 features of one token per thread).  A warp gives its share
+// of the accumulators back after its last load: gate/up both halves at once, down
+// one 128-feature half after the other.  Warps 10-13 are the fused dispatch
 // of the gate/up GEMM: they copy token rows (local, or P2P loads from the source
 // ranks over NVLink) into the sorted row buffer one 16-row granule at a time,
 // granules strided over the CTAs in row order, and count each granule's arrival;
@@ -522,7 +524,7 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
     // barrier that follows on the stream then covers them)
     __threadfence_system();
   } else {
-    // ---------------- epilogue: 8 (gate/up) or 12 (down) warps, one accumulator row (feature) per thread ----------------
+    // ---------------- epilogue: 8 (gate/up) or 12 (down) warps, each on 32 accumulator rows (features) ----------------
     const int ew = warp - kFirstEpilogueWarp;
     const int quarter = warp & 3;     // tensor-memory lanes 32*quarter .. +31
     const int cgroup = ew >> 2;       // which 16-column chunks this warp takes (c mod kChunkStride)

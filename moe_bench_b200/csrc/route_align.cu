@@ -7,7 +7,7 @@
 //    ids directly); this is the front end a caller with logits needs.
 //
 //  * align: stable counting sort of the flat assignment index n = token*k+kpos
-//    by local expert slot, every expert segment padded to 128 rows.  It
+//    by local expert slot, every expert segment padded to pad_rows rows.  It
 //    reproduces the slot order of the reference's schedule builder on one rank
 //    (tk_scheme.py:98-126, equal to the argsort key of tk_scheme.py:338-342)
 //    and replaces the moe_align_block_size step inside fused_experts

@@ -1,24 +1,31 @@
 """Small forwards launch their kernels chained (a kernel may start before the one ahead of it has
 ended).  Nothing may be seen early: inputs written on the stream just before the call, outputs read
-just after it, the same through a captured graph, and forwards on two streams at once."""
+just after it, the same through a captured graph, and forwards on two streams at once.  The output of
+each case is also compared with the oracle, since every run here takes the chained path."""
 
 import pytest
 import torch
 
 from moe_bench_b200 import problem as P
 from moe_bench_b200.plugin import get_implementation
+from oracle import moe_oracle as O
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
-# precision, tokens, experts: 16-bit; fp8 with tokens on the columns; fp8 128-row tiles; first and
-# last sizes of the one-block sort (4096 assignments) and of chaining (8192)
-CASES = [("bf16", 1, 64), ("fp16", 512, 16), ("bf16", 513, 16), ("bf16", 1025, 8), ("fp8", 3, 64), ("fp8", 200, 4),
-         ("fp8", 1024, 32)]
+# precision, tokens, experts, hidden, intermediate: 16-bit; fp8 with tokens on the columns; fp8 128-row
+# tiles; sorts of one block (up to 1024 assignments) and of several, last size of chaining (8192).  fp8
+# with tokens on the columns and a sort of several blocks has every kernel chained to the one ahead of it:
+# count, scatter, quantise, row gather, gate/up, down, combine.
+CASES = [("bf16", 1, 64, 1024, 512), ("fp16", 512, 16, 1024, 512), ("bf16", 513, 16, 1024, 512),
+         ("bf16", 1025, 8, 1024, 512), ("fp8", 3, 64, 1024, 512), ("fp8", 200, 4, 1024, 512),
+         ("fp8", 1024, 32, 1024, 512), ("bf16", 128, 32, 512, 256), ("bf16", 129, 32, 512, 256),
+         ("fp8", 129, 256, 512, 256), ("fp8", 600, 256, 256, 128), ("fp8", 600, 512, 512, 256),
+         ("fp8", 1024, 640, 256, 128)]
 
 
-def _setup(precision, tokens, experts, seed):
-    cfg = P.MoEBenchConfig(hidden_size=1024, intermediate_size=512, num_experts=experts, topk=min(8, experts),
+def _setup(precision, tokens, experts, seed, hidden=1024, intermediate=512):
+    cfg = P.MoEBenchConfig(hidden_size=hidden, intermediate_size=intermediate, num_experts=experts, topk=min(8, experts),
                            world_size=1, precision=P.Precision(precision), seed=seed, device=DEV)
     prob = P.make_problem(cfg, tokens)
     impl = get_implementation("b200")
@@ -33,9 +40,14 @@ def _variants(prob, n=4):
     return xs, ids
 
 
-@pytest.mark.parametrize("precision,tokens,experts", CASES)
-def test_inputs_written_on_the_stream(precision, tokens, experts):
-    impl, prob = _setup(precision, tokens, experts, 1)
+@pytest.mark.parametrize("precision,tokens,experts,hidden,intermediate", CASES)
+def test_inputs_written_on_the_stream(precision, tokens, experts, hidden, intermediate):
+    impl, prob = _setup(precision, tokens, experts, 1, hidden, intermediate)
+    first = impl.run(prob)
+    res = O.verify_output(precision, first, O.reference_moe(prob))
+    # three roundings to 8 (11) significand bits, 2^-9 (2^-12) each, relative to a sum of k terms; fp8 keeps
+    # bf16 activations and both sides quantise the same values
+    assert res.passed and res.rel_err < (1.5e-3 if precision == "fp16" else 1e-2), (res.message, res.rel_err)
     xs, ids = _variants(prob)
     want = []
     for x, i in zip(xs, ids):

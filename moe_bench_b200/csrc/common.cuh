@@ -243,6 +243,35 @@ __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, Wa
   }
 }
 
+// Warp-collective wait until counters[0 .. n) (n <= 32, in global memory, raised with fence +
+// atomicAdd by whoever wrote the data they stand for) have all reached `target`; the same answer
+// in all lanes.  Each lane acquires a counter of its own, and the vote that joins them orders no
+// memory: the __syncwarp does, so that on return the data of every counter is visible to every lane,
+// whichever of them reads it or issues the loads.
+template <int kPollsPerSleep, int kSleepNs>
+__device__ __forceinline__ bool wait_counters(const int* counters, int n, int target, WaitCtx& ctx, int where) {
+  const int lane = threadIdx.x & 31;
+  uint32_t spins = 0;
+  WaitClock clock;
+  while (true) {
+    int v = target;
+    if (lane < n) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(counters + lane) : "memory");
+    if (__all_sync(0xffffffffu, v >= target)) break;
+    if ((++spins & 0x3F) == 0) {
+      // warp-uniform decisions: the lanes read the flag and the timer at slightly different moments
+      const bool aborted = __any_sync(0xffffffffu, *ctx.abort_flag != 0);
+      const bool late = __any_sync(0xffffffffu, clock.expired(ctx));
+      if (aborted || late) {
+        if (!aborted && lane == 0) wait_give_up(ctx, where);
+        return false;
+      }
+    }
+    if (spins % kPollsPerSleep == 0) __nanosleep(kSleepNs);
+  }
+  __syncwarp();
+  return true;
+}
+
 // ---- programmatic dependent launch -----------------------------------------------
 // A kernel launched with launch_chained() may start while the kernel before it on the stream is
 // still running (once all of that kernel's blocks have called pdl_trigger() or exited).

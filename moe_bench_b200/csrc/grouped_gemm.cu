@@ -299,25 +299,7 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
       if (kMode == kGateUpSwiglu && disp.enabled) {
         // all 16-row granules of this token block must have been dispatched
         const int g0 = tc.row0 / kPad, ng = tc.ntok / kPad;  // ng <= 16
-        uint32_t spins = 0;
-        WaitClock clock;
-        while (true) {
-          int v = disp.granule_target;
-          if (lane < ng)
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(disp.granule_done + g0 + lane) : "memory");
-          if (__all_sync(0xffffffffu, v >= disp.granule_target)) break;
-          if ((++spins & 0x3F) == 0) {
-            // warp-uniform decisions: the lanes read the flag and the timer at slightly different moments
-            const bool aborted = __any_sync(0xffffffffu, *ctx.abort_flag != 0);
-            const bool late = __any_sync(0xffffffffu, clock.expired(ctx));
-            if (aborted || late) {
-              if (!aborted && lane == 0) wait_give_up(ctx, 6);
-              ok = false;
-              break;
-            }
-            __nanosleep(128);
-          }
-        }
+        ok = wait_counters<64, 128>(disp.granule_done + g0, ng, disp.granule_target, ctx, 6);
         if (!ok) break;
         // rows were written with ordinary stores by other SMs; the TMA engine reads them
         asm volatile("fence.proxy.async;" ::: "memory");

@@ -223,24 +223,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
       if (kMode == kGateUpSwiglu && disp.enabled) {
         // the eight 16-row granules of this token tile must have been dispatched
         const int g0 = tc.row0 / 16;
-        uint32_t spins = 0;
-        WaitClock clock;
-        while (true) {
-          int v = kFp8HelperWarps;
-          if (lane < kTileM / 16)
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(disp.granule_done + g0 + lane) : "memory");
-          if (__all_sync(0xffffffffu, v >= kFp8HelperWarps)) break;
-          if ((++spins & 0x3F) == 0) {
-            const bool aborted = __any_sync(0xffffffffu, *ctx.abort_flag != 0);
-            const bool late = __any_sync(0xffffffffu, clock.expired(ctx));
-            if (aborted || late) {
-              if (!aborted && lane == 0) wait_give_up(ctx, 6);
-              ok = false;
-              break;
-            }
-            __nanosleep(128);
-          }
-        }
+        ok = wait_counters<64, 128>(disp.granule_done + g0, kTileM / 16, kFp8HelperWarps, ctx, 6);
         if (!ok) break;
         // rows and scales were written with ordinary stores by other SMs; the TMA engine reads them
         asm volatile("fence.proxy.async;" ::: "memory");

@@ -215,7 +215,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_a,
         // first tile: the stages are empty and the weights depend on nothing but the schedule,
         // so they are requested before the wait for the tokens
         ahead = kStages < k_blocks ? kStages : k_blocks;
-        if (lane == 0)
+        if (elect_one())
           for (int kb = 0; kb < ahead; ++kb) load_weights(kb, kb);
         __syncwarp();
         if (args.early == kEarlyBeforePrevious) pdl_wait();

@@ -52,3 +52,13 @@ def test_a_vote_is_not_what_orders_the_rows(name):
 def test_the_kernels_that_wait_for_rows_are_known():
     waits = {os.path.basename(p) for p in glob.glob(os.path.join(mb_build.CSRC, "*.cu")) if "fence.proxy.async" in _source(os.path.basename(p))}
     assert waits == {"grouped_gemm.cu", "grouped_gemm_fp8.cu"}
+
+
+@pytest.mark.parametrize("name", GEMMS)
+def test_one_thread_issues_all_loads_of_a_barrier(name):
+    """Every call that arms a stage's barrier or loads into it is behind the same choice of a lane."""
+    text = _source(name)
+    calls = [m.start() for m in re.finditer(r"\bload_weights\(kb", text)]
+    assert len(calls) == 2
+    guards = {re.findall(r"if \((lane == 0|elect_one\(\))\)", text[:at])[-1] for at in calls}
+    assert len(guards) == 1

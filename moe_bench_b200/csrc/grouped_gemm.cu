@@ -463,23 +463,7 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w,
       const int nb = tail->tb_prefix[lo + 1] - tail->tb_prefix[lo];
       const int per = (blocks16 + nb - 1) / nb;
       const int tb = tail->tb_prefix[lo] + (g - tail->prefix[lo]) / per;
-      uint32_t spins = 0;
-      WaitClock clock;
-      while (true) {
-        int v;
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(push.block_done + tb) : "memory");
-        if (v >= target) break;
-        if ((++spins & 0x3F) == 0) {
-          const bool aborted = __any_sync(0xffffffffu, *ctx.abort_flag != 0);
-          const bool late = __any_sync(0xffffffffu, clock.expired(ctx));
-          if (aborted || late) {
-            if (!aborted && lane == 0) wait_give_up(ctx, 7);
-            ok = false;
-            break;
-          }
-        }
-        __nanosleep(256);
-      }
+      ok = wait_counters<1, 256>(push.block_done + tb, 1, target, ctx, 7);
       if (!ok) break;
       for (int i = pw; i < kPad; i += kPushWarps) {
         const int n = __ldg(args.sorted_ids + g * kPad + i);

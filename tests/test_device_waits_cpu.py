@@ -62,3 +62,13 @@ def test_one_thread_issues_all_loads_of_a_barrier(name):
     assert len(calls) == 2
     guards = {re.findall(r"if \((lane == 0|elect_one\(\))\)", text[:at])[-1] for at in calls}
     assert len(guards) == 1
+
+
+@pytest.mark.parametrize("name", GEMMS)
+def test_no_lane_leaves_a_polling_loop_alone(name):
+    """A lane that breaks out on what it read itself would be missing from the full-mask votes of the
+    lanes that read the counter a moment earlier: all polling is done by the wait whose exit is a vote."""
+    assert "ld.acquire" not in _source(name)
+    common = _source("common.cuh")
+    body = _block(common, common.index("bool wait_counters("))
+    assert re.findall(r"if \(([^;{}]*)\) break;", body) == ["__all_sync(0xffffffffu, v >= target)"]

@@ -184,9 +184,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, WaitCtx
   const bool ok = mbar_wait_lane(bar, parity, ctx, where);
   return __all_sync(0xffffffffu, ok);
 }
-// One poll, this lane's answer, for a wait that comes later: the answer of a poll takes about 110 cycles
-// whether the phase is complete or not, so a loop polls for its next step before it is through with
-// this one.  (test_wait: a try_wait may suspend the thread.)
+// One poll, this lane's answer, for a wait that comes later: a loop that polls for its next step before
+// it is through with this one has the answer (58 cycles in a loop of polls, phase complete or not) by
+// the time it waits.  (test_wait: a try_wait may suspend the thread.)
 __device__ __forceinline__ uint32_t mbar_peek(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -206,17 +206,7 @@ __device__ __forceinline__ bool mbar_wait_peeked(uint32_t peeked, uint32_t bar, 
 }
 // One poll, no waiting; the same answer in all lanes.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred P;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, P;\n\t"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return __all_sync(0xffffffffu, ok != 0);
+  return __all_sync(0xffffffffu, mbar_peek(bar, parity) != 0);
 }
 __device__ __forceinline__ bool mbar_wait_lane(uint32_t bar, uint32_t parity, WaitCtx& ctx, int where) {
   uint32_t spins = 0;
